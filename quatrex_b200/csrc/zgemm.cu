@@ -7,46 +7,61 @@
 // warp-level DMMA (mma.sync m16n8k4 .f64) -- on B200 the FP64 tensor and
 // vector rates are equal, and DMMA needs 8x fewer issue slots than DFMA.
 //
-// Complex arithmetic uses the 3M (Gauss) form on interleaved operands: one
-// 16-byte shared-memory load yields the real and the imaginary fragment of an
-// element, and the three real MMAs  Ar Br,  Ai Bi  and  (Ar + Ai)(Br + Bi)
-// give  Re = p1 - p2  and  Im = p3 - p1 - p2  in the epilogue.
+// Complex arithmetic uses the 3M (Gauss) form on interleaved operands: the
+// three real MMAs  Ar Br,  Ai Bi  and  (Ar + Ai)(Br + Bi)  give
+// Re = p1 - p2  and  Im = p3 - p1 - p2  in the epilogue. A conjugated operand
+// flips the sign of its imaginary part in the sums and of p2 (compile time).
 // Conjugate-transposed operands are staged k-major so every fragment load
-// stays conflict-free (strides = 4 mod 8 or 2 mod 8 in 16-byte units), and
-// conjugation is a compile-time sign flip.
+// stays conflict-free (strides = 4 mod 8 or 2 mod 8 in 16-byte units).
 //
-// Tiles: CTA 64x64 complex, 4 warps of 32x32, BK = 8 complex per stage,
-// 4-stage cp.async pipeline (zero-filled at the matrix edges). The epilogue
-// fuses up to four scaled (optionally conjugate-transposed) addends, a
-// conjugate-transposed second store and a second output with its own
-// addends, so chains like  S = A_jj - Sigma - P A_ij  or
-// X_ij = -X_ii A X_jj  with  X_ji = -X_ij^H  are one launch. It runs through
-// a padded shared-memory tile: transposed operands are read and written with
-// lanes along rows, the others with lanes along columns (coalesced both ways,
-// many independent loads in flight).
+// The DMMA pipe is the bound (36.4-37.0 TFLOP/s from registers alone), so the
+// design keeps it fed:
+//  * CTA tile 32 x 32, four warps of 16 x 16, four CTAs per SM. The 64 x 64
+//    tile of an earlier version (two CTAs, 254 registers) shared more operands
+//    per load, but eight warps per SM left the pipe idle 17 % of the time, and
+//    its few large tiles filled the last wave badly: 256^3 x 148 487 -> 468 us,
+//    256^3 x 64 244 -> 208 us, 288^3 x 24 178 -> 119 us, 128^3 x 16 24 -> 12.5
+//    us, 160^3 x 100 141 -> 84 us; with an addend 519 -> 478 us at 256^3 x 148.
+//    64 x 32 and 32 x 64 tiles at three CTAs per SM and k-slices of 16 measured
+//    the same or slower at every size. 86 % DMMA + 4 % for the sums in ncu.
+//  * Per k-step of 4 the three passes p1, p2, p3 are issued back to back; the
+//    real parts of the next step are loaded (8-byte loads) right after p1,
+//    which frees their registers, the imaginary parts after p2, so a load has
+//    a pass of MMAs to land. The stage barrier (cp.async, STAGES buffers of BK)
+//    sits after p1 of a stage's last step: by then the stage has been read, so
+//    its buffer is refilled at once.
+//  * The epilogue works on the accumulator fragments: one store covers 128
+//    contiguous bytes of a row (lanes tq), its transposed counterpart 128 bytes
+//    of a column (lanes g), so the addends, the second output and the
+//    conjugate-transposed second store are coalesced in either orientation
+//    without a shared-memory tile.
+//  * Warps whose 16 x 16 (or 16 x 8) part lies outside the matrix issue no
+//    MMAs: a block of 200 costs 13 x 12.5 of them instead of 16 x 16.
 #include "common.cuh"
 
 namespace qtx {
 namespace {
 
-constexpr int BM = 64;
-constexpr int BN = 64;
+constexpr int THREADS = 128;    // 2 x 2 warps
+constexpr int NT = 2;           // 16 x 8 fragments per warp, side by side
+constexpr int WM = 16;          // rows and
+constexpr int WN = 8 * NT;      // columns of a warp tile
+constexpr int BM = 2 * WM;
+constexpr int BN = 2 * WN;
 constexpr int BK = 8;
 constexpr int STAGES = 4;
-constexpr int THREADS = 128;
-constexpr int WM = 32;
-constexpr int WN = 32;
-constexpr int MT = WM / 16;  // m16 tiles per warp
-constexpr int NT = WN / 8;   // n8 tiles per warp
+constexpr int CTAS_PER_SM = 4;
 
 // Shared-memory strides (complex elements).
-constexpr int S_MK = BK + 4;  // [row][k] layouts: stride = 4 mod 8
-constexpr int S_KM = BM + 2;  // [k][row] layouts: stride = 2 mod 8
-constexpr int A_MK_SIZE = BM * S_MK;
-constexpr int A_KM_SIZE = BK * S_KM;
-constexpr int B_NK_SIZE = BN * S_MK;
-constexpr int B_KN_SIZE = BK * (BN + 2);
-constexpr int TS = BN + 1;  // epilogue tile row stride (complex): 1 mod 8 in 16-byte units
+constexpr int S_RK = BK + 4;  // [row][k] layouts: stride = 4 mod 8
+template <int R>
+constexpr int s_kr() {  // [k][row] layouts: stride = 2 mod 8
+  return R + 2;
+}
+template <int R, bool RK>
+constexpr int stage_elems() {
+  return RK ? R * S_RK : BK * s_kr<R>();
+}
 
 __device__ __forceinline__ void mma_f64(double (&c)[4], double a0, double a1, double b0) {
   asm volatile(
@@ -60,290 +75,302 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, bool pred) {
+__device__ __forceinline__ void cp_async16(uint32_t smem, const void* gmem, bool pred) {
   const int bytes = pred ? 16 : 0;
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem_u32(smem)), "l"(gmem),
-               "r"(bytes));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(smem), "l"(gmem), "r"(bytes));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
+// The barrier of the CTA, reached from main loops of different active size
+// (each warp runs one of them).
+__device__ __forceinline__ void cta_barrier() { asm volatile("bar.sync 0, %0;\n" ::"n"(THREADS) : "memory"); }
 
-// Loads one BK slice of op(A) (OPA = 0: A is M x K; 1: A is K x M) or of
-// op(B) (OPB = 0: B is K x N; 1: B is N x K) into shared memory.
-template <int OP, bool IS_A>
-__device__ __forceinline__ void load_tile(z64* sm, const z64* g, int64_t ld, int rows_total,
-                                          int cols_total, int r0, int k0, int tid) {
-  // "rows" = M (for A) or N (for B); the tile spans 64 rows x BK k-values.
-  if (OP == (IS_A ? 0 : 1)) {
-    // Global rows are the M/N index, k contiguous: [row][k] layout.
-#pragma unroll
-    for (int it = 0; it < (64 * BK) / THREADS; ++it) {
-      const int idx = tid + it * THREADS;
-      const int r = idx / BK;
-      const int k = idx % BK;
-      const int gr = r0 + r, gk = k0 + k;
-      const bool ok = (gr < rows_total) && (gk < cols_total);
-      const z64* src = ok ? g + (int64_t)gr * ld + gk : g;
-      cp_async16(sm + r * S_MK + k, src, ok);
+__device__ __forceinline__ double lds64(uint32_t addr) {
+  double v;
+  asm volatile("ld.shared.f64 %0, [%1];\n" : "=d"(v) : "r"(addr));
+  return v;
+}
+
+// Copies BK-wide slices of one operand tile of R rows (M for op(A), N for
+// op(B)) into the stages. RK: the global rows are the M / N index, k is
+// contiguous ([row][k] in shared memory); otherwise the rows are the k index
+// ([k][row]). Out-of-range elements are zero-filled.
+template <int R, bool RK>
+struct Loader {
+  const z64* base;  // in range: the address of a zero-filled element
+  const z64* p;     // this thread's element of the next slice
+  int64_t ld;
+  int rows, k;  // rows left from this thread's row; its k within a slice
+  uint32_t off;
+
+  __device__ __forceinline__ Loader(const z64* g, int64_t ld_, int total, int r0, int tid) {
+    base = g;
+    ld = ld_;
+    if (RK) {
+      const int r = tid / BK;
+      k = tid % BK;
+      rows = total - (r0 + r);
+      p = g + (int64_t)(r0 + r) * ld + k;
+      off = (uint32_t)(r * S_RK + k) * 16u;
+    } else {
+      const int r = tid % R;
+      k = tid / R;
+      rows = total - (r0 + r);
+      p = g + (int64_t)k * ld + (r0 + r);
+      off = (uint32_t)(k * s_kr<R>() + r) * 16u;
     }
-  } else {
-    // Global rows are the k index, M/N contiguous: [k][row] layout.
+  }
+  // krem: k values left from the start of this slice.
+  __device__ __forceinline__ void load(uint32_t sm, int krem) {
+    constexpr int ITERS = R * BK / THREADS;
 #pragma unroll
-    for (int it = 0; it < (64 * BK) / THREADS; ++it) {
-      const int idx = tid + it * THREADS;
-      const int k = idx / 64;
-      const int r = idx % 64;
-      const int gr = r0 + r, gk = k0 + k;
-      const bool ok = (gr < rows_total) && (gk < cols_total);
-      const z64* src = ok ? g + (int64_t)gk * ld + gr : g;
-      cp_async16(sm + k * S_KM + r, src, ok);
+    for (int it = 0; it < ITERS; ++it) {
+      if (RK) {
+        constexpr int RS = THREADS / BK;
+        const bool ok = it * RS < rows && k < krem;
+        cp_async16(sm + off + it * RS * S_RK * 16, ok ? p + (int64_t)(it * RS) * ld : base, ok);
+      } else {
+        constexpr int KS = THREADS / R;
+        const bool ok = 0 < rows && k + it * KS < krem;
+        cp_async16(sm + off + it * KS * s_kr<R>() * 16, ok ? p + (int64_t)(it * KS) * ld : base, ok);
+      }
+    }
+    p += RK ? BK : BK * ld;
+  }
+};
+
+constexpr int kMaxGroup = 4;
+struct KernelArgs {
+  int count;
+  GemmDesc d[kMaxGroup];
+};
+
+struct Acc {
+  double p1[NT][4], p2[NT][4], p3[NT][4];
+};
+
+// All k-steps of a warp with NTA active fragments (0: it only copies and
+// synchronises).
+template <int OPA, int OPB, int NTA>
+__device__ __forceinline__ void main_loop(Acc& acc, uint32_t as, uint32_t bs, uint32_t a_off, uint32_t b_off,
+                                          Loader<BM, OPA == 0>& la, Loader<BN, OPB == 1>& lb, int K, int KT) {
+  constexpr int A_BYTES = stage_elems<BM, OPA == 0>() * 16;
+  constexpr int B_BYTES = stage_elems<BN, OPB == 1>() * 16;
+  constexpr int NA = NTA > 0 ? NTA : 1;
+  constexpr bool ON = NTA > 0;
+  // byte offsets of a row of A / column of B and of a k
+  constexpr int A_ROW = (OPA == 0 ? S_RK : 1) * 16, A_K = (OPA == 0 ? 1 : s_kr<BM>()) * 16;
+  constexpr int B_ROW = (OPB == 1 ? S_RK : 1) * 16, B_K = (OPB == 1 ? 1 : s_kr<BN>()) * 16;
+  double ar[2], ai[2], br[NA], bi[NA];
+  auto load_re = [&](uint32_t a, uint32_t b, int kk) {
+    ar[0] = lds64(a + (uint32_t)(kk * A_K));
+    ar[1] = lds64(a + (uint32_t)(8 * A_ROW + kk * A_K));
+#pragma unroll
+    for (int j = 0; j < NTA; ++j) br[j] = lds64(b + (uint32_t)(j * 8 * B_ROW + kk * B_K));
+  };
+  auto load_im = [&](uint32_t a, uint32_t b, int kk) {
+    ai[0] = lds64(a + (uint32_t)(kk * A_K + 8));
+    ai[1] = lds64(a + (uint32_t)(8 * A_ROW + kk * A_K + 8));
+#pragma unroll
+    for (int j = 0; j < NTA; ++j) bi[j] = lds64(b + (uint32_t)(j * 8 * B_ROW + kk * B_K + 8));
+  };
+  cp_async_wait<STAGES - 1>();
+  cta_barrier();
+  uint32_t a_cur = as + a_off, b_cur = bs + b_off;
+  if (ON) {
+    load_re(a_cur, b_cur, 0);
+    load_im(a_cur, b_cur, 0);
+  }
+  int st = 0, krem = K - STAGES * BK;
+  for (int kt = 0; kt < KT; ++kt) {
+#pragma unroll
+    for (int h = 0; h < BK / 4; ++h) {
+      const bool last = h == BK / 4 - 1;
+      double sa[2], sb[NA];
+      if (ON) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) sa[q] = OPA ? ar[q] - ai[q] : ar[q] + ai[q];
+#pragma unroll
+        for (int j = 0; j < NTA; ++j) sb[j] = OPB ? br[j] - bi[j] : br[j] + bi[j];
+#pragma unroll
+        for (int j = 0; j < NTA; ++j) mma_f64(acc.p1[j], ar[0], ar[1], br[j]);
+      }
+      uint32_t an = a_cur, bn = b_cur;
+      if (last) {
+        // This stage has been read by every warp once they all arrive; the
+        // next one has landed.
+        cp_async_wait<STAGES - 2>();
+        cta_barrier();
+        if (krem > 0) {
+          la.load(as + st * A_BYTES, krem);
+          lb.load(bs + st * B_BYTES, krem);
+        }
+        cp_async_commit();
+        krem -= BK;
+        st = st + 1 == STAGES ? 0 : st + 1;
+        an = as + a_off + st * A_BYTES;
+        bn = bs + b_off + st * B_BYTES;
+      }
+      const int kn = last ? 0 : 4 * (h + 1);
+      if (ON) {
+        load_re(an, bn, kn);
+#pragma unroll
+        for (int j = 0; j < NTA; ++j) mma_f64(acc.p2[j], ai[0], ai[1], bi[j]);
+        load_im(an, bn, kn);
+#pragma unroll
+        for (int j = 0; j < NTA; ++j) mma_f64(acc.p3[j], sa[0], sa[1], sb[j]);
+      }
+      a_cur = an;
+      b_cur = bn;
     }
   }
 }
 
-struct KernelArgs {
-  GemmDesc d;
-};
+// Element (r, c) of op(X) of an addend, zero outside the matrix.
+__device__ __forceinline__ z64 addend_at(const z64* p, int64_t rs, int64_t cs, double sg, bool ok, int r, int c) {
+  const z64 x = ok ? p[r * rs + c * cs] : make_double2(0.0, 0.0);
+  return make_double2(x.x, sg * x.y);
+}
 
 template <int OPA, int OPB>
-__global__ void __launch_bounds__(THREADS, 2) zgemm_kernel(const KernelArgs args) {
-  const GemmDesc& d = args.d;
+__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) zgemm_kernel(const __grid_constant__ KernelArgs args) {
+  constexpr int A_BYTES = stage_elems<BM, OPA == 0>() * 16;
+  constexpr int B_BYTES = stage_elems<BN, OPB == 1>() * 16;
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  z64* smem = reinterpret_cast<z64*>(smem_raw);
-  constexpr int A_SIZE = (OPA == 0) ? A_MK_SIZE : A_KM_SIZE;
-  constexpr int B_SIZE = (OPB == 1) ? B_NK_SIZE : B_KN_SIZE;
-  z64* As = smem;
-  z64* Bs = smem + STAGES * A_SIZE;
+  const uint32_t as = smem_u32(smem_raw);
+  const uint32_t bs = as + STAGES * A_BYTES;
 
   const int tid = threadIdx.x;
   const int lane = tid & 31;
-  const int warp = tid >> 5;
   const int g = lane >> 2;
   const int tq = lane & 3;
-  const int wm0 = (warp >> 1) * WM;
-  const int wn0 = (warp & 1) * WN;
   const int m0 = blockIdx.y * BM;
   const int n0 = blockIdx.x * BN;
-  const int M = d.M, N = d.N, K = d.K;
+  const int M = args.d[0].M, N = args.d[0].N, K = args.d[0].K;
   const int KT = (K + BK - 1) / BK;
+  const int64_t batch = args.d[0].batch;
 
-  for (int64_t b = blockIdx.z; b < d.batch; b += gridDim.z) {
+  for (int64_t z = blockIdx.z; z < batch * args.count; z += gridDim.z) {
+    const int set = args.count == 1 ? 0 : (int)(z / batch);
+    const int64_t b = args.count == 1 ? z : z - set * batch;
+    const GemmDesc& d = args.d[set];
     if (d.active != nullptr && d.active[b] == 0) continue;
+    // Edge tiles leave their last warps idle: alternate which schedulers
+    // host those.
+    const int warp = (tid >> 5) ^ ((z & 1) ? 3 : 0);
+    const int wm0 = (warp >> 1) * WM;
+    const int wn0 = (warp & 1) * WN;
     const z64* Ag = d.a_ptrs ? d.a_ptrs[b] : at<const z64>(d.A, b);
     const z64* Bg = d.b_ptrs ? d.b_ptrs[b] : at<const z64>(d.B, b);
 
-    // 3M (Gauss) products: p1 = sum ar br, p2 = sum ai bi,
-    // p3 = sum (ar + ai)(br + bi); Re = p1 - p2, Im = p3 - p1 - p2.
-    double p1[MT][NT][4], p2[MT][NT][4], p3[MT][NT][4];
+    Acc acc;
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
+    for (int j = 0; j < NT; ++j)
 #pragma unroll
-      for (int j = 0; j < NT; ++j)
+      for (int q = 0; q < 4; ++q) acc.p1[j][q] = acc.p2[j][q] = acc.p3[j][q] = 0.0;
+    if (KT > 0) {
+      Loader<BM, OPA == 0> la(Ag, d.A.ld, M, m0, tid);
+      Loader<BN, OPB == 1> lb(Bg, d.B.ld, N, n0, tid);
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          p1[i][j][q] = 0.0;
-          p2[i][j][q] = 0.0;
-          p3[i][j][q] = 0.0;
-        }
-
-    // Prologue.
-#pragma unroll
-    for (int s = 0; s < STAGES - 1; ++s) {
-      if (s < KT) {
-        load_tile<OPA, true>(As + s * A_SIZE, Ag, d.A.ld, M, K, m0, s * BK, tid);
-        load_tile<OPB, false>(Bs + s * B_SIZE, Bg, d.B.ld, N, K, n0, s * BK, tid);
-      }
-      cp_async_commit();
-    }
-
-    for (int kt = 0; kt < KT; ++kt) {
-      cp_async_wait<STAGES - 2>();
-      __syncthreads();
-      {
-        const int nk = kt + STAGES - 1;
-        if (nk < KT) {
-          const int st = nk % STAGES;
-          load_tile<OPA, true>(As + st * A_SIZE, Ag, d.A.ld, M, K, m0, nk * BK, tid);
-          load_tile<OPB, false>(Bs + st * B_SIZE, Bg, d.B.ld, N, K, n0, nk * BK, tid);
+      for (int s = 0; s < STAGES; ++s) {
+        if (s < KT) {
+          la.load(as + s * A_BYTES, K - s * BK);
+          lb.load(bs + s * B_BYTES, K - s * BK);
         }
         cp_async_commit();
       }
-      const z64* as = As + (kt % STAGES) * A_SIZE;
-      const z64* bs = Bs + (kt % STAGES) * B_SIZE;
-#pragma unroll
-      for (int kk = 0; kk < BK; kk += 4) {
-        double ar[MT][2], ai[MT][2], sa[MT][2];
-#pragma unroll
-        for (int i = 0; i < MT; ++i) {
-          const int r = wm0 + i * 16 + g;
-          z64 v0, v1;
-          if (OPA == 0) {
-            v0 = as[r * S_MK + kk + tq];
-            v1 = as[(r + 8) * S_MK + kk + tq];
-          } else {
-            v0 = as[(kk + tq) * S_KM + r];
-            v1 = as[(kk + tq) * S_KM + r + 8];
-          }
-          ar[i][0] = v0.x;
-          ar[i][1] = v1.x;
-          ai[i][0] = (OPA == 1) ? -v0.y : v0.y;
-          ai[i][1] = (OPA == 1) ? -v1.y : v1.y;
-          sa[i][0] = ar[i][0] + ai[i][0];
-          sa[i][1] = ar[i][1] + ai[i][1];
-        }
-        double br[NT], bi[NT], sb[NT];
-#pragma unroll
-        for (int j = 0; j < NT; ++j) {
-          const int c = wn0 + j * 8 + g;
-          z64 v;
-          if (OPB == 1)
-            v = bs[c * S_MK + kk + tq];
-          else
-            v = bs[(kk + tq) * (BN + 2) + c];
-          br[j] = v.x;
-          bi[j] = (OPB == 1) ? -v.y : v.y;
-          sb[j] = br[j] + bi[j];
-        }
-        // Three passes over the 2x4 tiles: the products feeding one
-        // accumulator are 8 independent MMAs apart.
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-          for (int j = 0; j < NT; ++j) mma_f64(p1[i][j], ar[i][0], ar[i][1], br[j]);
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-          for (int j = 0; j < NT; ++j) mma_f64(p2[i][j], ai[i][0], ai[i][1], bi[j]);
-#pragma unroll
-        for (int i = 0; i < MT; ++i)
-#pragma unroll
-          for (int j = 0; j < NT; ++j) mma_f64(p3[i][j], sa[i][0], sa[i][1], sb[j]);
-      }
+      const uint32_t a_off =
+          OPA == 0 ? (uint32_t)((wm0 + g) * S_RK + tq) * 16u : (uint32_t)(tq * s_kr<BM>() + wm0 + g) * 16u;
+      const uint32_t b_off =
+          OPB == 1 ? (uint32_t)((wn0 + g) * S_RK + tq) * 16u : (uint32_t)(tq * s_kr<BN>() + wn0 + g) * 16u;
+      const int cols = M > m0 + wm0 ? N - n0 - wn0 : 0;  // columns this warp has to compute
+      if (cols > 8)
+        main_loop<OPA, OPB, 2>(acc, as, bs, a_off, b_off, la, lb, K, KT);
+      else if (cols > 0)
+        main_loop<OPA, OPB, 1>(acc, as, bs, a_off, b_off, la, lb, K, KT);
+      else
+        main_loop<OPA, OPB, 0>(acc, as, bs, a_off, b_off, la, lb, K, KT);
+      cp_async_wait<0>();
+      if (gridDim.z < batch * args.count) cta_barrier();  // the stages serve the next entry
     }
-    cp_async_wait<0>();
-    __syncthreads();
 
-    // Epilogue through a padded shared-memory tile (it reuses the stage
-    // buffers) so that global reads and writes are coalesced in either
-    // orientation. Phase A (fragment layout, lanes mostly along rows):
-    // alpha * acc + the conjugate-transposed addends -> tile.
-    z64* tile = smem;
+    // Epilogue on the fragments: element (j, q) is row r0 + 8 (q / 2), column
+    // c0 + 8 j + q % 2.
+    const int r0 = m0 + wm0 + g, c0 = n0 + wn0 + 2 * tq;
+    auto row = [&](int q) { return r0 + ((q >> 1) << 3); };
+    auto col = [&](int j, int q) { return c0 + j * 8 + (q & 1); };
+    auto inside = [&](int j, int q) { return row(q) < M && col(j, q) < N; };
+    z64 v[NT][4];
 #pragma unroll
-    for (int i = 0; i < MT; ++i)
+    for (int j = 0; j < NT; ++j)
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const double x1 = acc.p1[j][q], x2 = acc.p2[j][q], x3 = acc.p3[j][q];
+        v[j][q] = zmul(d.alpha, (OPA ^ OPB) ? make_double2(x1 + x2, x3 - (x1 - x2))
+                                            : make_double2(x1 - x2, x3 - (x1 + x2)));
+      }
+    // Adds coef op(D) of addend t to w, all loads first.
+    auto add = [&](int t, z64(&w)[NT][4]) {
+      const Addend& ad = d.add[t];
+      const z64* p = (t == 0 && d.d_ptrs) ? d.d_ptrs[b] : at<const z64>(ad.m, b);
+      const int64_t rs = ad.conj_trans ? 1 : ad.m.ld, cs = ad.conj_trans ? ad.m.ld : 1;
+      const double sg = ad.conj_trans ? -1.0 : 1.0;
+      z64 x[NT][4];
 #pragma unroll
       for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-          const int rl = wm0 + i * 16 + g + ((q >> 1) << 3);
-          const int cl = wn0 + j * 8 + 2 * tq + (q & 1);
-          const double re = p1[i][j][q] - p2[i][j][q];
-          const double im = p3[i][j][q] - (p1[i][j][q] + p2[i][j][q]);
-          tile[rl * TS + cl] = zmul(d.alpha, make_double2(re, im));
-        }
-    for (int t = 0; t < d.nadd; ++t) {
-      const Addend& ad = d.add[t];
-      if (!ad.conj_trans) continue;
-      const z64* p = (t == 0 && d.d_ptrs) ? d.d_ptrs[b] : at<const z64>(ad.m, b);
-      z64 x[MT][NT][4];  // all loads first: many in flight, no aliasing stalls
+        for (int q = 0; q < 4; ++q) x[j][q] = addend_at(p, rs, cs, sg, inside(j, q), row(q), col(j, q));
 #pragma unroll
-      for (int i = 0; i < MT; ++i)
+      for (int j = 0; j < NT; ++j)
 #pragma unroll
-        for (int j = 0; j < NT; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int r = m0 + wm0 + i * 16 + g + ((q >> 1) << 3);
-            const int c = n0 + wn0 + j * 8 + 2 * tq + (q & 1);
-            x[i][j][q] = (r < M && c < N) ? p[(int64_t)c * ad.m.ld + r] : make_double2(0.0, 0.0);
-          }
-#pragma unroll
-      for (int i = 0; i < MT; ++i)
-#pragma unroll
-        for (int j = 0; j < NT; ++j)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int rl = wm0 + i * 16 + g + ((q >> 1) << 3);
-            const int cl = wn0 + j * 8 + 2 * tq + (q & 1);
-            tile[rl * TS + cl] = zfma(ad.coef, zconj(x[i][j][q]), tile[rl * TS + cl]);
-          }
-    }
-    __syncthreads();
-    // Phase B (lanes along columns): the other addends, C3 and C.
-    constexpr int PER = BM * BN / THREADS;  // elements per thread
-    for (int t = 0; t < d.nadd; ++t) {
-      const Addend& ad = d.add[t];
-      if (ad.conj_trans) continue;
-      const z64* p = (t == 0 && d.d_ptrs) ? d.d_ptrs[b] : at<const z64>(ad.m, b);
-      z64 x[PER];  // all loads first: many in flight, no aliasing stalls
-#pragma unroll
-      for (int k = 0; k < PER; ++k) {
-        const int e = tid + k * THREADS;
-        const int r = m0 + e / BN, c = n0 + e % BN;
-        x[k] = (r < M && c < N) ? p[(int64_t)r * ad.m.ld + c] : make_double2(0.0, 0.0);
-      }
-#pragma unroll
-      for (int k = 0; k < PER; ++k) {
-        const int e = tid + k * THREADS;
-        const int rl = e / BN, cl = e % BN;
-        tile[rl * TS + cl] = zfma(ad.coef, x[k], tile[rl * TS + cl]);
-      }
-    }
+        for (int q = 0; q < 4; ++q) w[j][q] = zfma(ad.coef, x[j][q], w[j][q]);
+    };
+    for (int t = 0; t < d.nadd; ++t) add(t, v);
     if (!d.C3.null()) {
-#pragma unroll 4
-      for (int e = tid; e < BM * BN; e += THREADS) {
-        const int rl = e / BN, cl = e % BN;
-        const int r = m0 + rl, c = n0 + cl;
-        if (r >= M || c >= N) continue;
-        z64 v3 = zmul(d.scale3, tile[rl * TS + cl]);
-        for (int t = d.nadd; t < d.nadd + d.nadd3; ++t) {
-          const Addend& ad = d.add[t];
-          const z64* p = at<const z64>(ad.m, b);
-          const z64 x = ad.conj_trans ? zconj(p[(int64_t)c * ad.m.ld + r]) : p[(int64_t)r * ad.m.ld + c];
-          v3 = zfma(ad.coef, x, v3);
-        }
-        at<z64>(d.C3, b)[(int64_t)r * d.C3.ld + c] = v3;
-      }
+      z64 w[NT][4];
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q) w[j][q] = zmul(d.scale3, v[j][q]);
+      for (int t = d.nadd; t < d.nadd + d.nadd3; ++t) add(t, w);
+      z64* out = at<z64>(d.C3, b);
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (inside(j, q)) out[(int64_t)row(q) * d.C3.ld + col(j, q)] = w[j][q];
     }
     if (!d.C.null()) {
       z64* out = d.c_ptrs ? d.c_ptrs[b] : at<z64>(d.C, b);
-#pragma unroll 8
-      for (int e = tid; e < BM * BN; e += THREADS) {
-        const int rl = e / BN, cl = e % BN;
-        const int r = m0 + rl, c = n0 + cl;
-        if (r < M && c < N) out[(int64_t)r * d.C.ld + c] = tile[rl * TS + cl];
-      }
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (inside(j, q)) out[(int64_t)row(q) * d.C.ld + col(j, q)] = v[j][q];
     }
-    // Phase C (lanes along rows): the conjugate-transposed second store,
-    // after every thread's phase-B updates of the tile.
     if (!d.C2.null()) {
-      __syncthreads();
-      z64* out2 = at<z64>(d.C2, b);
-#pragma unroll 8
-      for (int e = tid; e < BM * BN; e += THREADS) {
-        const int rl = e % BM, cl = e / BM;
-        const int r = m0 + rl, c = n0 + cl;
-        if (r < M && c < N) out2[(int64_t)c * d.C2.ld + r] = zmul(d.coef2, zconj(tile[rl * TS + cl]));
-      }
+      z64* out = at<z64>(d.C2, b);
+#pragma unroll
+      for (int j = 0; j < NT; ++j)
+#pragma unroll
+        for (int q = 0; q < 4; ++q)
+          if (inside(j, q)) out[(int64_t)col(j, q) * d.C2.ld + row(q)] = zmul(d.coef2, zconj(v[j][q]));
     }
-    __syncthreads();  // the tile aliases the stage buffers of the next entry
   }
 }
 
 template <int OPA, int OPB>
-int launch(const GemmDesc& d, cudaStream_t s) {
-  constexpr int A_SIZE = (OPA == 0) ? A_MK_SIZE : A_KM_SIZE;
-  constexpr int B_SIZE = (OPB == 1) ? B_NK_SIZE : B_KN_SIZE;
-  constexpr size_t stages = STAGES * (A_SIZE + B_SIZE) * sizeof(z64);
-  constexpr size_t tile = (size_t)BM * TS * sizeof(z64);
-  constexpr size_t smem = stages > tile ? stages : tile;
-  QTX_CHECK_CUDA(cudaFuncSetAttribute(zgemm_kernel<OPA, OPB>,
-                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((d.N + BN - 1) / BN, (d.M + BM - 1) / BM,
-            (unsigned)(d.batch < 65535 ? d.batch : 65535));
-  KernelArgs args{d};
-  ProfScope prof(QTX_KERNEL_ZGEMM, 8.0 * d.M * d.N * (double)d.K * (double)d.batch, s);
+int launch(const KernelArgs& args, cudaStream_t s) {
+  const GemmDesc& d = args.d[0];
+  constexpr size_t smem =
+      (size_t)STAGES * (stage_elems<BM, OPA == 0>() + stage_elems<BN, OPB == 1>()) * sizeof(z64);
+  static_assert(smem <= 48 * 1024, "no opt-in of dynamic shared memory needed");
+  const int64_t z = d.batch * args.count;
+  dim3 grid((d.N + BN - 1) / BN, (d.M + BM - 1) / BM, (unsigned)(z < 65535 ? z : 65535));
+  ProfScope prof(QTX_KERNEL_ZGEMM, 8.0 * d.M * d.N * (double)d.K * (double)z, s);
   zgemm_kernel<OPA, OPB><<<grid, THREADS, smem, s>>>(args);
   QTX_CHECK_LAUNCH();
   return QTX_OK;
@@ -401,12 +428,15 @@ int zgemm(const GemmDesc& d, cudaStream_t s) {
     void* scr = oz_bound(&bytes);
     if (scr != nullptr) return zgemm_oz(dd, gemm_slices(), scr, bytes, s);
   }
+  KernelArgs args;
+  args.count = 1;
+  args.d[0] = dd;
   const int key = dd.opA * 2 + dd.opB;
   switch (key) {
-    case 0: return launch<0, 0>(dd, s);
-    case 1: return launch<0, 1>(dd, s);
-    case 2: return launch<1, 0>(dd, s);
-    default: return launch<1, 1>(dd, s);
+    case 0: return launch<0, 0>(args, s);
+    case 1: return launch<0, 1>(args, s);
+    case 2: return launch<1, 0>(args, s);
+    default: return launch<1, 1>(args, s);
   }
 }
 
