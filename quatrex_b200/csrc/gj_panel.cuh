@@ -2,18 +2,31 @@
 // columns), shared by the one-CTA (zinv.cu) and the cluster
 // (zinv_cluster.cu) batched inverses.
 //
-// The panel stays in registers for all of its columns, so one column step
-// touches shared memory only for the pivot search partials and the
-// broadcast pivot row. Per column k:
-//   pivot  p = argmax_{r >= k} |Re| + |Im| of column k (lowest row on ties,
-//          the izamax measure of LAPACK that numpy.linalg.inv uses);
-//   the threads of row p publish 1 / x_pk and the scaled pivot row, the
-//   threads of row k the old row k;
-//   row k <- scaled pivot row; row p <- old row k; every row r != k is
-//   eliminated: x_rc -= x_rk * prow_c (c != k), x_rk <- -x_rk / x_pk.
-// Afterwards the panel holds the transform T of the panel (T = [A_KK^-1 ;
-// -A_RK A_KK^-1] in block form) and pivrow[k0 .. k0 + nbp) the pivot rows.
-// Two CTA barriers per column; every thread of the CTA must call it.
+// One thread holds one row of the panel for all of its columns, so a column
+// step touches shared memory only for the pivot search partials and the
+// broadcast pivot row. Rows are not interchanged: each thread tracks the
+// position its row would have after LAPACK's interchanges. Per column k:
+//   pivot  p = argmax_{pos >= k} |Re| + |Im| of column k (lowest position on
+//          ties, the izamax measure of LAPACK that numpy.linalg.inv uses);
+//   the pivot row's thread publishes the row q and takes position k, the
+//   row at position k takes position p;
+//   with m = x_rk / x_pk every other row is eliminated, x_rc -= m q_c
+//   (c != k), x_rk <- -m, and the pivot row becomes q / x_pk.
+// Afterwards the rows, stored at their positions, hold the transform T of the
+// panel (T = [A_KK^-1 ; -A_RK A_KK^-1] in block form).
+//
+// A column step is a chain of latencies and of instructions that every warp
+// issues: the search compares the measures as integers (one redux of the high
+// words and a ballot, a slow path only if they tie) instead of five shuffle
+// rounds; the candidate's value travels with the search, so that every thread
+// forms 1 / x_pk itself while the pivot row is published; and the loop over the
+// columns is rolled. Cycles per column, factorization alone, at n = 64 / 256 /
+// 512: 1120 / 1455 / 2010 (two lanes to a row, five shuffle rounds and an
+// unrolled loop took about 3000 at n = 256). Measured beside it: two or four
+// lanes to a row with every warp publishing its candidate row and one barrier
+// 1130 / 2340 / - (a row written by one or two lanes costs as much as one
+// written by all), whole columns in a warp with the multipliers published
+// 1100 / 2440 / 4840; not inlined, 25 % slower in the inverse at n = 64.
 #pragma once
 
 #include "common.cuh"
@@ -34,7 +47,7 @@ __device__ __forceinline__ z64 gj_recip_scaled(z64 z) {
   int e;
   frexp(mx, &e);
   const double xs = ldexp(z.x, -e), ys = ldexp(z.y, -e);
-  const double m = fma(xs, xs, ys * ys);
+  const double m = fma(xs, xs, __dmul_rn(ys, ys));
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(m));
 #pragma unroll
@@ -53,7 +66,7 @@ __device__ __forceinline__ z64 gj_recip(z64 z) {
   const int e = eb - 1022;                                         // frexp's exponent of mx
   const double s = __longlong_as_double((long long)(1023 - e) << 52);  // 2^-e
   const double xs = z.x * s, ys = z.y * s;
-  const double m = fma(xs, xs, ys * ys);
+  const double m = fma(xs, xs, __dmul_rn(ys, ys));
   double y;
   asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(m));
 #pragma unroll
@@ -63,112 +76,127 @@ __device__ __forceinline__ z64 gj_recip(z64 z) {
 
 __device__ __forceinline__ double gj_abs1(z64 z) { return fabs(z.x) + fabs(z.y); }
 
-// Panel of 16 columns, n <= 256, 512 threads: the two lanes 2i and 2i + 1
-// of warp w hold row 16 w + i, columns 0-7 and 8-15 respectively, so a row's
-// value in the pivot column reaches its partner lane with one shuffle.
-// load(r, c) / store(r, c, v): panel element access (r < n, c < nbp).
-// prow_s, rowk_s: 16 shared complex each; red_v / red_i: 16 shared entries
-// each; sing: shared int, set to k + 1 at the first zero pivot if still 0.
-template <class Load, class Store>
-__device__ __forceinline__ void gj_factor_panel16(int n, int k0, int nbp, Load load, Store store, int* pivrow,
-                                                  z64* prow_s, z64* rowk_s, double* red_v, int* red_i,
-                                                  int* sing) {
-  constexpr int NB = 16, H = 8, W = 16;
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int h = lane & 1;                       // which 8 columns
-  const int r = warp * 16 + (lane >> 1);        // which row
-  const bool live = r < n;
-  z64 v[H];
-#pragma unroll
-  for (int c = 0; c < H; ++c) v[c] = (live && h * H + c < nbp) ? load(r, h * H + c) : make_double2(0.0, 0.0);
-#pragma unroll
-  for (int kk = 0; kk < NB; ++kk) {
-    if (kk >= nbp) break;
-    const int k = k0 + kk;
-    const int hk = kk / H, ck = kk % H;  // compile-time after unrolling
-    // this row's value in column kk (held by the lane with h == hk)
-    const z64 mine = (h == hk) ? v[ck] : make_double2(0.0, 0.0);
-    z64 xk;
-    xk.x = __shfl_xor_sync(0xffffffffu, mine.x, 1);
-    xk.y = __shfl_xor_sync(0xffffffffu, mine.y, 1);
-    if (h == hk) xk = mine;
-    double best = -1.0;
-    int besti = k;
-    if (live && r >= k && h == hk) {
-      best = gj_abs1(xk);
-      besti = r;
-    }
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) {
-      const double ov = __shfl_xor_sync(0xffffffffu, best, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, besti, off);
-      if (ov > best || (ov == best && oi < besti)) {
-        best = ov;
-        besti = oi;
-      }
-    }
-    if (lane == 0) {
-      red_v[warp] = best;
-      red_i[warp] = besti;
-    }
-    __syncthreads();
-    // every warp reduces the W partials with shuffles (lanes >= W repeat them)
-    best = red_v[lane & (W - 1)];
-    besti = red_i[lane & (W - 1)];
-#pragma unroll
-    for (int off = W / 2; off > 0; off >>= 1) {
-      const double ov = __shfl_xor_sync(0xffffffffu, best, off);
-      const int oi = __shfl_xor_sync(0xffffffffu, besti, off);
-      if (ov > best || (ov == best && oi < besti)) {
-        best = ov;
-        besti = oi;
-      }
-    }
-    const int p = besti;
-    if (r == p) {
-      const z64 d = gj_recip(xk);
-#pragma unroll
-      for (int c = 0; c < H; ++c) prow_s[h * H + c] = (h * H + c == kk) ? d : zmul(v[c], d);
-    }
-    if (r == k) {
-#pragma unroll
-      for (int c = 0; c < H; ++c) rowk_s[h * H + c] = v[c];
-    }
-    if (tid == 0) {
-      pivrow[k] = p;
-      if (best <= 0.0 && *sing == 0) *sing = k + 1;
-    }
-    __syncthreads();
-    // (the next column's partials, prow_s and rowk_s are written after its
-    // first barrier, when every thread has read these)
-    if (!live) continue;
-    if (r == k) {
-#pragma unroll
-      for (int c = 0; c < H; ++c) v[c] = prow_s[h * H + c];
-      continue;
-    }
-    z64 f = xk;
-    if (r == p) {  // row p receives the old row k
-#pragma unroll
-      for (int c = 0; c < H; ++c) v[c] = rowk_s[h * H + c];
-      f = rowk_s[kk];
-    }
-    const z64 dpiv = prow_s[kk];
-#pragma unroll
-    for (int c = 0; c < H; ++c) {
-      if (h * H + c == kk) continue;
-      const z64 qc = prow_s[h * H + c];
-      v[c] = make_double2(v[c].x - (f.x * qc.x - f.y * qc.y), v[c].y - (f.x * qc.y + f.y * qc.x));
-    }
-    if (h == hk) {
-      const z64 m = zmul(f, dpiv);
-      v[ck] = make_double2(-m.x, -m.y);
-    }
+// a b and v - m q with the roundings spelled out: every instantiation of the
+// factorization gives the same bits, so one block's inverse does not depend on
+// the path that the batch size selects.
+__device__ __forceinline__ z64 gj_mul(z64 a, z64 b) {
+  return make_double2(fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.x, b.y, __dmul_rn(a.y, b.x)));
+}
+__device__ __forceinline__ z64 gj_eliminate(z64 v, z64 m, z64 q) {
+  return make_double2(fma(-m.x, q.x, fma(m.y, q.y, v.x)), fma(-m.x, q.y, fma(-m.y, q.x, v.y)));
+}
+
+// Shared memory of gj_factor_panel.
+template <int NB>
+struct GjPanelSmem {
+  z64 q[2][NB];                // pivot row, double-buffered by column parity
+  z64 val[16];                 // per-warp candidate: value,
+  unsigned long long key[16];  // measure + 1 (0: none),
+  int pos[16];                 // position
+};
+
+// The lane holding the largest key (lowest position on ties) of the warp.
+// Every lane takes part in every step of the search.
+__device__ __forceinline__ int gj_best_lane(unsigned long long key, int pos) {
+  const unsigned hi = (unsigned)(key >> 32);
+  const unsigned m1 = __reduce_max_sync(0xffffffffu, hi);
+  unsigned cand = __ballot_sync(0xffffffffu, hi == m1);
+  if ((cand & (cand - 1)) != 0) {
+    const unsigned lo = hi == m1 ? (unsigned)key : 0u;
+    const unsigned m2 = __reduce_max_sync(0xffffffffu, lo);
+    const bool c2 = hi == m1 && (unsigned)key == m2;
+    const int m3 = __reduce_min_sync(0xffffffffu, c2 ? pos : 0x7fffffff);
+    cand = __ballot_sync(0xffffffffu, c2 && pos == m3);
   }
-  if (live) {
+  return __ffs(cand) - 1;
+}
+
+// Factors an n x nbp panel (nbp <= NB, n <= 512); the first ceil(n / 32) warps
+// of the CTA take part and the others return at once (named barrier 1).
+// load(r, c) / store(r, c, v): panel element access (r < n, c < nbp), the same
+// memory or not (a barrier separates loads and stores); moved(r, pos), once per
+// row after that barrier: row r ends at position pos; pivot(k, p), by one
+// thread: position p was chosen for column k. sing: shared int, set to k + 1 at
+// the first zero pivot if still 0.
+template <int NB, class Load, class Store, class Moved, class Pivot>
+__device__ __forceinline__ void gj_factor_panel(int n, int k0, int nbp, Load load, Store store, Moved moved,
+                                                Pivot pivot, int* sing) {
+  __shared__ GjPanelSmem<NB> sm;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int W = (n + 31) >> 5;
+  if (warp >= W) return;
+  const int bar_threads = W * 32;
+  auto barrier = [&]() {
+    if (W > 1)
+      asm volatile("bar.sync 1, %0;\n" ::"r"(bar_threads) : "memory");
+    else
+      __syncwarp();
+  };
+  const bool live = tid < n;
+  int pos = live ? tid : 0x7fffffff;
+  z64 v[NB];
 #pragma unroll
-    for (int c = 0; c < H; ++c)
-      if (h * H + c < nbp) store(r, h * H + c, v[c]);
+  for (int c = 0; c < NB; ++c) v[c] = (live && c < nbp) ? load(tid, c) : make_double2(0.0, 0.0);
+  // The columns rotate through the registers: column k is always v[0], and
+  // the eliminated column enters at v[NB - 1]. The loop therefore stays
+  // rolled: unrolled over the columns its straight-line code (5 KB a column)
+  // is fetched anew for every panel and costs more than the arithmetic.
+#pragma unroll 1
+  for (int kk = 0; kk < nbp; ++kk) {
+    const int k = k0 + kk;
+    const bool mine = live && pos >= k;
+    {
+      const double a = gj_abs1(v[0]);
+      // NaN compares false: such a row is never chosen
+      const unsigned long long key = (mine && a >= 0.0) ? (unsigned long long)__double_as_longlong(a) + 1 : 0ull;
+      const int tie = mine ? pos : 0x7fffffff;
+      if (lane == gj_best_lane(key, tie)) {
+        sm.key[warp] = key;
+        sm.pos[warp] = tie;
+        sm.val[warp] = v[0];
+      }
+    }
+    barrier();
+    const unsigned long long wkey = lane < W ? sm.key[lane & 15] : 0ull;
+    const int wpos = lane < W ? sm.pos[lane & 15] : 0x7fffffff;
+    const int wl = gj_best_lane(wkey, wpos);
+    const int p = __shfl_sync(0xffffffffu, wpos, wl);
+    const z64 xp = sm.val[wl];
+    const bool piv = live && pos == p;
+    z64* q = sm.q[kk & 1];
+    if (piv) {
+#pragma unroll
+      for (int c = 1; c < NB; ++c) q[c] = v[c];
+    }
+    const z64 d = gj_recip(xp);
+    z64 m = gj_mul(v[0], d);
+    if (piv) {
+      // the scaled pivot row q / x_pk as 0 - (-1 / x_pk) q
+      pivot(k, p);
+      if (sm.key[wl] <= 1ull && *sing == 0) *sing = k + 1;
+#pragma unroll
+      for (int c = 1; c < NB; ++c) v[c] = make_double2(0.0, 0.0);
+      m = make_double2(-d.x, -d.y);
+      pos = k;
+    } else if (pos == k) {
+      pos = p;
+    }
+    barrier();
+#pragma unroll
+    for (int c = 1; c < NB; ++c) {
+      v[c - 1] = gj_eliminate(v[c], m, q[c]);
+      if (c % 5 == 0) asm volatile("" ::: "memory");  // bounds the loads in flight (registers)
+    }
+    v[NB - 1] = make_double2(-m.x, -m.y);
+  }
+  barrier();  // every load of the panel (and of the last pivot row) is done
+  if (live) {
+    moved(tid, pos);
+#pragma unroll
+    for (int c = 0; c < NB; ++c) {
+      const int col = c + nbp < NB ? c + nbp : c + nbp - NB;  // after nbp rotations
+      if (col < nbp) store(pos, col, v[c]);
+    }
   }
 }
 

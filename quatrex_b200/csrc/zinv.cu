@@ -360,8 +360,8 @@ int launch(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* activ
 }
 
 // ---------------------------------------------------------------------------
-// Second generation (n <= 720): the same Gauss-Jordan with the same pivot
-// rule, reorganised so that the trailing update runs without barriers.
+// One CTA per matrix for 512 < n <= 720: the same Gauss-Jordan with the same
+// pivot rule, reorganised so that the trailing update runs without barriers.
 // Per panel of NB columns:
 //   1. stage the n x NB panel (odd row stride: row-per-thread access is
 //      conflict-free) and factor it (one barrier pair per column, the next
@@ -395,18 +395,9 @@ struct Smem2 {
   }
 };
 
-// Column split (csplit = C > 1, launched as clusters of C CTAs, one matrix
-// per cluster): every CTA of the cluster factors each panel itself (the
-// same arithmetic on the same data, so the same transform and pivots) and
-// applies it to its own range of whole panels' columns; the panel's columns
-// are written back by the CTA that owns them. A cluster barrier after each
-// panel orders the owner's writes before the next panel's loads (read
-// through L2), and the final row gather is split by rows. The serial panel
-// factorization stays, the update is divided by C: for small batches, C SMs
-// per matrix instead of one.
 template <int NB>
 __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatRef A, MatRef X, int* info,
-                                                      const int* active, int csplit) {
+                                                      const int* active) {
   using S = Smem2<NB>;
   // Column block of the row-interchange pass: all 2 NB affected rows of CW
   // columns fit T2 x PV registers.
@@ -429,51 +420,26 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, tq = lane & 3;
-  const int rank = (int)(blockIdx.x % csplit);
-  // this CTA's columns [c_lo, c_hi): whole panels
-  auto cbound = [&](int q) {
-    const int v = (int)(((int64_t)n * q / csplit + NB - 1) / NB) * NB;
-    return v < n ? v : n;
-  };
-  const int c_lo = cbound(rank), c_hi = cbound(rank + 1), cw = c_hi - c_lo;
-  auto cluster_sync = [&]() {
-    if (csplit > 1) cg::this_cluster().sync();
-  };
-
-  for (int64_t b = blockIdx.x / csplit; b < batch; b += gridDim.x / csplit) {
+  for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
     if (active != nullptr && active[b] == 0) continue;
     const z64* a = at<const z64>(A, b);
     z64* x = at<z64>(X, b);
     const int64_t ldx = X.ld;
     if (a != x) {
-      for (int64_t idx = tid; idx < (int64_t)n * cw; idx += T2) {
-        const int r = (int)(idx / cw), c = c_lo + (int)(idx % cw);
+      for (int64_t idx = tid; idx < (int64_t)n * n; idx += T2) {
+        const int r = (int)(idx / n), c = (int)(idx % n);
         x[(int64_t)r * ldx + c] = a[(int64_t)r * A.ld + c];
       }
     }
     if (tid == 0) s_sing = 0;
     __syncthreads();
-    cluster_sync();
 
     for (int k0 = 0; k0 < n; k0 += NB) {
       const int nbp = min(NB, n - k0);
-      // 1. Stage the panel and factor it: in registers for 16-column panels
-      //    of at most 256 rows (two lanes per row), through shared memory
-      //    otherwise.
-      if (NB == 16 && n <= 256) {
+      // 1. Stage the panel and factor it.
       for (int idx = tid; idx < n * NB; idx += T2) {
         const int r = idx / NB, c = idx % NB;
-        P[r * PS + c] = (c < nbp) ? __ldcg(&x[(int64_t)r * ldx + k0 + c]) : make_double2(0.0, 0.0);
-      }
-      __syncthreads();
-      gj_factor_panel16(
-          n, k0, nbp, [&](int r, int c) { return P[r * PS + c]; },
-          [&](int r, int c, z64 v) { P[r * PS + c] = v; }, pivrow, prow, rowk, red_v, red_i, &s_sing);
-      __syncthreads();
-      } else {
-      for (int idx = tid; idx < n * NB; idx += T2) {
-        const int r = idx / NB, c = idx % NB;
-        P[r * PS + c] = (c < nbp) ? __ldcg(&x[(int64_t)r * ldx + k0 + c]) : make_double2(0.0, 0.0);
+        P[r * PS + c] = (c < nbp) ? x[(int64_t)r * ldx + k0 + c] : make_double2(0.0, 0.0);
       }
       __syncthreads();
       double best = -1.0;
@@ -550,7 +516,6 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
           }
         }
       }
-      }
       // 2. The panel's interchanges as a permutation of the affected rows:
       //    row aff_row[a] receives the old content of row aff_src[a].
       if (tid == 0) {
@@ -580,8 +545,7 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
       }
       __syncthreads();
       const int na = s_na;
-      const bool pin = k0 >= c_lo && k0 < c_hi;  // the panel lies in this CTA's columns
-      const int oc = cw - (pin ? nbp : 0);       // this CTA's columns outside the panel
+      const int oc = n - nbp;  // columns outside the panel
       // In column blocks of CW: all affected rows of a column move within
       // one block (read all, barrier, write all).
       for (int cb = 0; cb < oc; cb += CW) {
@@ -591,7 +555,7 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
           const int li = tid + u * T2;
           const int aa = li / CW, cc = cb + li % CW;
           if (aa < na && cc < oc) {
-            const int c = c_lo + cc + ((pin && c_lo + cc >= k0) ? nbp : 0);
+            const int c = cc + (cc >= k0 ? nbp : 0);
             v[u] = x[(int64_t)aff_src[aa] * ldx + c];
           }
         }
@@ -601,7 +565,7 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
           const int li = tid + u * T2;
           const int aa = li / CW, cc = cb + li % CW;
           if (aa < na && cc < oc) {
-            const int c = c_lo + cc + ((pin && c_lo + cc >= k0) ? nbp : 0);
+            const int c = cc + (cc >= k0 ? nbp : 0);
             x[(int64_t)aff_row[aa] * ldx + c] = v[u];
           }
         }
@@ -611,7 +575,7 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
       const int ny = YS - 2;  // columns of whole tiles; those >= n stay zero
       for (int idx = tid; idx < NB * ny; idx += T2) {
         const int kk = idx / ny, c = idx % ny;
-        Y[kk * YS + c] = (kk < nbp && c >= c_lo && c < c_hi && (c < k0 || c >= k0 + nbp))
+        Y[kk * YS + c] = (kk < nbp && c < n && (c < k0 || c >= k0 + nbp))
                              ? x[(int64_t)(k0 + kk) * ldx + c]
                              : make_double2(0.0, 0.0);
       }
@@ -621,7 +585,7 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
       for (int mt = warp; mt < mtiles; mt += W2) {
         const int r0 = mt * 16;
         // A fragments of this slice for all k (the panel transform rows).
-        for (int j0 = c_lo; j0 < c_hi; j0 += 8 * JN) {
+        for (int j0 = 0; j0 < n; j0 += 8 * JN) {
           if (j0 >= k0 && j0 + 8 * JN <= k0 + nbp) continue;  // inside the panel
           double cre[JN][4], cim[JN][4];
 #pragma unroll
@@ -672,15 +636,12 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
         }
       }
       __syncthreads();
-      // 5. The panel transform back into X[:, K] (by the CTA owning K).
-      if (pin) {
-        for (int idx = tid; idx < n * nbp; idx += T2) {
-          const int r = idx / nbp, c = idx % nbp;
-          x[(int64_t)r * ldx + k0 + c] = P[r * PS + c];
-        }
+      // 5. The panel transform back into X[:, K].
+      for (int idx = tid; idx < n * nbp; idx += T2) {
+        const int r = idx / nbp, c = idx % nbp;
+        x[(int64_t)r * ldx + k0 + c] = P[r * PS + c];
       }
       __syncthreads();
-      cluster_sync();
     }
 
     // Undo the column permutation: swaps applied from the last pivot back.
@@ -697,16 +658,260 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
     }
     __syncthreads();
     // Row-wise gather through the (now free) panel buffer: PS rows fit.
-    // Rows rank, rank + C, ... of a column split (read through L2: the
-    // other CTAs wrote their columns).
     const int nbufs = PS < W2 ? PS : W2;
     if (warp < nbufs) {
       z64* rowbuf = P + (size_t)warp * n;
-      for (int r = rank + warp * csplit; r < n; r += nbufs * csplit) {
-        for (int c = lane; c < n; c += 32) rowbuf[c] = __ldcg(&x[(int64_t)r * ldx + colsrc[c]]);
+      for (int r = warp; r < n; r += nbufs) {
+        for (int c = lane; c < n; c += 32) rowbuf[c] = x[(int64_t)r * ldx + colsrc[c]];
         __syncwarp();
         for (int c = lane; c < n; c += 32) x[(int64_t)r * ldx + c] = rowbuf[c];
         __syncwarp();
+      }
+    }
+    if (tid == 0 && info != nullptr && s_sing != 0 && info[b] == 0) info[b] = s_sing;
+    __syncthreads();
+  }
+}
+
+template <int NB>
+int launch2(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s) {
+  const size_t smem = Smem2<NB>::bytes(n);
+  if (smem > 227 * 1024) {
+    set_error("zinv: block size too large for the shared-memory panel");
+    return QTX_ERR_UNSUPPORTED;
+  }
+  QTX_CHECK_CUDA(
+      cudaFuncSetAttribute(zinv2_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  const unsigned grid = (unsigned)(batch < 131072 ? batch : 131072);
+  ProfScope prof(QTX_KERNEL_ZINV, 8.0 * (double)n * n * n * (double)batch, s);
+  zinv2_kernel<NB><<<grid, T2, smem, s>>>(n, batch, A, X, info, active);
+  QTX_CHECK_LAUNCH();
+  return QTX_OK;
+}
+
+// ---------------------------------------------------------------------------
+// n <= 512: one thread-block cluster of C CTAs per matrix (C = 1 at full
+// batches), the CTAs splitting the columns; panels of 16 columns.
+// Per panel:
+//   1. every CTA factors the panel itself (gj_panel.cuh; the same arithmetic on
+//      the same data, so the same transform and pivots) -- no broadcast;
+//      rows are not interchanged, the factorization only says where they go;
+//   2. the pivot rows Y of this CTA's columns are staged, and the owner of the
+//      panel's columns writes the transform T there;
+//   3. all row slices but the pivots' own are updated, X[r, J] <- X[src(r), J]
+//      + T[r, :] Y[:, J] (DMMA): src(r) is r, or the row of K that LAPACK's
+//      interchanges would have moved to r, so the interchange costs no pass of
+//      its own. The tiles of 16 x 16 are dealt to the warps evenly;
+//   4. after a barrier (slices read rows of K) the pivots' slice becomes T Y.
+// A cluster barrier ends the panel when C > 1 (other CTAs read the next panel
+// through L2). Finally the columns are gathered in the order of the pivoting.
+//
+// RES: the matrix stays in shared memory from load to store (n <= 100, one
+// CTA); otherwise each panel is a pass over the matrix in L2 / HBM, which at
+// 256 x 256 x 148 moves 5 GB a launch, about half of its time.
+struct Smem3 {
+  static constexpr int NB = 16;
+  __host__ __device__ static int rows(int n) { return (n + 15) & ~15; }
+  // Columns of the widest CTA of a C-way split (whole panels).
+  __host__ __device__ static int bound(int n, int C, int q) {
+    const int v = (int)(((int64_t)n * q / C + NB - 1) / NB) * NB;
+    return v < n ? v : n;
+  }
+  __host__ __device__ static int ys(int n, int C) {  // Y row stride: 2 mod 8 in 16-byte units
+    int w = 0;
+    for (int q = 0; q < C; ++q) {
+      const int c = bound(n, C, q + 1) - bound(n, C, q);
+      w = c > w ? c : w;
+    }
+    return rows(w) + 2;
+  }
+  __host__ __device__ static int xs(int n) { return n | 1; }  // resident row stride (odd)
+  static size_t bytes(int n, int C, bool res) {
+    size_t s = (size_t)rows(n) * NB * sizeof(z64) + (size_t)NB * ys(n, C) * sizeof(z64);
+    if (res) s += (size_t)n * xs(n) * sizeof(z64);
+    return s + (size_t)4 * rows(n) * sizeof(int);
+  }
+};
+
+// Element (r, c) of the panel transform in shared memory: conflict-free both
+// for a thread per row and for the DMMA fragments.
+__device__ __forceinline__ int tix(int r, int c) { return r * 16 + (c ^ (((r & 1) << 2) | ((r >> 1) & 3))); }
+
+template <int TH, int RPL, bool RES>
+__global__ void __launch_bounds__(TH, 512 / TH) zinv3_kernel(int n, int64_t batch, MatRef A, MatRef X, int* info,
+                                                            const int* active, int csplit) {
+  using S = Smem3;
+  constexpr int NB = S::NB, WARPS3 = TH / 32;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  const int np = S::rows(n), YS = S::ys(n, csplit), XS = S::xs(n);
+  z64* T = reinterpret_cast<z64*>(smem_raw);
+  z64* Y = T + (size_t)np * NB;
+  z64* Xs = Y + (size_t)NB * YS;
+  int* srcrow = reinterpret_cast<int*>(RES ? Xs + (size_t)n * XS : Xs);
+  int* orig = srcrow + np;      // 2 x np: original row of each position
+  int* colsrc = orig + 2 * np;  // np
+  __shared__ int s_sing;
+
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int g = lane >> 2, tq = lane & 3;
+  const int rank = (int)(blockIdx.x % csplit);
+  const int c_lo = S::bound(n, csplit, rank), c_hi = S::bound(n, csplit, rank + 1), cw = c_hi - c_lo;
+  const int mtiles = np / 16, ntiles = (cw + 15) / 16;
+  auto cluster_sync = [&]() {
+    if (csplit > 1) cg::this_cluster().sync();
+  };
+
+  for (int64_t b = blockIdx.x / csplit; b < batch; b += gridDim.x / csplit) {
+    if (active != nullptr && active[b] == 0) continue;
+    const z64* a = at<const z64>(A, b);
+    z64* xg = at<z64>(X, b);
+    z64* x = RES ? Xs : xg;
+    const int64_t ldx = RES ? XS : X.ld;
+    if (RES || a != xg || A.ld != X.ld) {
+      for (int idx = tid; idx < n * cw; idx += TH) {
+        const int r = idx / cw, c = c_lo + idx % cw;
+        x[r * ldx + c] = a[(int64_t)r * A.ld + c];
+      }
+    }
+    for (int r = tid; r < n; r += TH) orig[r] = r;
+    if (tid == 0) s_sing = 0;
+    __syncthreads();
+    cluster_sync();
+
+    int cur = 0;
+    for (int k0 = 0; k0 < n; k0 += NB) {
+      const int nbp = min(NB, n - k0), kt = k0 / NB;
+      // 1. Factor the panel.
+      gj_factor_panel<NB>(
+          n, k0, nbp,
+          [=](int r, int c) { return RES ? x[r * ldx + k0 + c] : __ldcg(&x[r * ldx + k0 + c]); },
+          [=](int r, int c, z64 v) { T[tix(r, c)] = v; },
+          [=](int r, int pos) {
+            srcrow[pos] = r;
+            orig[(cur ^ 1) * np + pos] = orig[cur * np + r];
+          },
+          [](int, int) {}, &s_sing);
+      cur ^= 1;
+      __syncthreads();
+      // 2. Pivot rows of this CTA's other columns; the transform into X[:, K].
+      const bool pin = k0 >= c_lo && k0 < c_hi;
+      for (int kk = warp; kk < NB; kk += WARPS3) {
+        const z64* xr = kk < nbp ? x + srcrow[k0 + kk] * ldx + c_lo : nullptr;
+        const int p0 = k0 - c_lo, p1 = p0 + nbp;  // the panel's columns: not used
+#pragma unroll 4
+        for (int j = lane; j < YS - 2; j += 32)
+          Y[kk * YS + j] = (xr != nullptr && j < cw && (j < p0 || j >= p1)) ? xr[j] : make_double2(0.0, 0.0);
+      }
+      {
+        const int c = tid % NB;
+        if (c >= nbp) {  // columns of T that the factorization left unwritten
+          for (int r = tid / NB; r < n; r += TH / NB) T[tix(r, c)] = make_double2(0.0, 0.0);
+        } else if (pin) {
+#pragma unroll 4
+          for (int r = tid / NB; r < n; r += TH / NB) x[r * ldx + k0 + c] = T[tix(r, c)];
+        }
+      }
+      __syncthreads();
+      // 3./4. Update of one 16 x 16 tile at row slice mt, local columns j0.
+      z64 t0[NB / 4], t1[NB / 4];  // this slice's rows of T, DMMA fragments
+      auto load_t = [&](int mt) {
+#pragma unroll
+        for (int k4 = 0; k4 < NB; k4 += 4) {
+          t0[k4 / 4] = T[tix(mt * 16 + g, k4 + tq)];
+          t1[k4 / 4] = T[tix(mt * 16 + g + 8, k4 + tq)];
+        }
+      };
+      auto update = [&](int mt, int j0, const z64* s0, const z64* s1) {
+        double cre[2][4], cim[2][4];
+        const int cl = j0 + 2 * tq;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const z64* sr = (q >> 1) ? s1 : s0;
+            const int cc = cl + j * 8 + (q & 1);
+            const z64 v = (sr != nullptr && cc < cw) ? sr[cc] : make_double2(0.0, 0.0);
+            cre[j][q] = v.x;
+            cim[j][q] = v.y;
+          }
+#pragma unroll
+        for (int k4 = 0; k4 < NB; k4 += 4) {
+          const z64 v0 = t0[k4 / 4], v1 = t1[k4 / 4];
+          z64 y[2];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) y[j] = Y[(k4 + tq) * YS + j0 + j * 8 + g];
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            mma_f64(cre[j], v0.x, v1.x, y[j].x);
+            mma_f64(cim[j], v0.x, v1.x, y[j].y);
+          }
+#pragma unroll
+          for (int j = 0; j < 2; ++j) {
+            mma_f64(cre[j], -v0.y, -v1.y, y[j].y);
+            mma_f64(cim[j], v0.y, v1.y, y[j].x);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+          for (int q = 0; q < 4; ++q) {
+            const int r = mt * 16 + g + ((q >> 1) << 3), cc = cl + j * 8 + (q & 1);
+            if (r < n && cc < cw) x[r * ldx + c_lo + cc] = make_double2(cre[j][q], cim[j][q]);
+          }
+      };
+      // Tiles outside the panel's columns, dealt evenly in row-slice order.
+      const int pt = pin ? (k0 - c_lo) / 16 : ntiles, nt = ntiles - (pin ? 1 : 0);
+      const int total = (mtiles - 1) * nt;
+      const int u0 = (int)((int64_t)total * warp / WARPS3), u1 = (int)((int64_t)total * (warp + 1) / WARPS3);
+      int last = -1;
+      const z64 *s0 = nullptr, *s1 = nullptr;
+      for (int u = u0; u < u1; ++u) {
+        int mt = u / nt, jt = u % nt;
+        if (mt >= kt) ++mt;
+        if (jt >= pt) ++jt;
+        if (mt != last) {
+          last = mt;
+          load_t(mt);
+          const int ra = mt * 16 + g;
+          s0 = ra < n ? x + srcrow[ra] * ldx + c_lo : nullptr;
+          s1 = ra + 8 < n ? x + srcrow[ra + 8] * ldx + c_lo : nullptr;
+        }
+        update(mt, jt * 16, s0, s1);
+      }
+      __syncthreads();
+      if (warp < nt) {
+        load_t(kt);
+        for (int u = warp; u < nt; u += WARPS3) update(kt, (u >= pt ? u + 1 : u) * 16, nullptr, nullptr);
+      }
+      __syncthreads();
+      cluster_sync();
+    }
+
+    // Position s holds original row orig[s], so column s of the result is
+    // column orig[s] of the inverse. Rows rank, rank + C, ... are gathered
+    // (through L2: the other CTAs wrote their columns).
+    for (int s = tid; s < n; s += TH) colsrc[orig[cur * np + s]] = s;
+    __syncthreads();
+    if (RES) {
+      for (int idx = tid; idx < n * n; idx += TH) {
+        const int r = idx / n, c = idx % n;
+        xg[(int64_t)r * X.ld + c] = x[r * ldx + colsrc[c]];
+      }
+    } else {
+      // Each warp holds a whole row in registers between reading and writing.
+      for (int r = rank + warp * csplit; r < n; r += WARPS3 * csplit) {
+        z64 v[RPL];  // n <= 32 RPL
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) {
+          const int c = lane + 32 * i;
+          if (c < n) v[i] = __ldcg(&x[r * ldx + colsrc[c]]);
+        }
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < RPL; ++i) {
+          const int c = lane + 32 * i;
+          if (c < n) x[r * ldx + c] = v[i];
+        }
       }
     }
     if (tid == 0 && rank == 0 && info != nullptr && s_sing != 0 && info[b] == 0) info[b] = s_sing;
@@ -716,86 +921,95 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
   }
 }
 
-template <int NB>
-int launch2(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s,
-            int csplit = 1) {
-  const size_t smem = Smem2<NB>::bytes(n);
-  if (smem > 227 * 1024) {
-    set_error("zinv: block size too large for the shared-memory panel");
-    return QTX_ERR_UNSUPPORTED;
-  }
-  QTX_CHECK_CUDA(
-      cudaFuncSetAttribute(zinv2_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+template <int TH, int RPL, bool RES>
+int configure3(int n, int64_t batch, int c, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, cudaStream_t s) {
+  const size_t smem = Smem3::bytes(n, c, RES);
+  QTX_CHECK_CUDA(cudaFuncSetAttribute(zinv3_kernel<TH, RPL, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      (int)smem));
   const int64_t mats = batch < 131072 ? batch : 131072;
-  ProfScope prof(QTX_KERNEL_ZINV, 8.0 * (double)n * n * n * (double)batch, s);
-  if (csplit <= 1) {
-    zinv2_kernel<NB><<<(unsigned)mats, T2, smem, s>>>(n, batch, A, X, info, active, 1);
-    QTX_CHECK_LAUNCH();
-    return QTX_OK;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(mats * csplit), 1, 1);
-  cfg.blockDim = dim3(T2, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = (unsigned)csplit;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, zinv2_kernel<NB>, n, batch, A, X, info, active, csplit));
+  *cfg = {};
+  cfg->gridDim = dim3((unsigned)(mats * c), 1, 1);
+  cfg->blockDim = dim3(TH, 1, 1);
+  cfg->dynamicSmemBytes = smem;
+  cfg->stream = s;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = (unsigned)c;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg->attrs = attr;
+  cfg->numAttrs = 1;
   return QTX_OK;
 }
 
-// Column split for n <= 400 (16-column panels): the largest C in {1, 2, 4, 8}
-// with batch x C within the SM count, at least 32 columns per CTA, and all
-// batch clusters co-resident (cudaOccupancyMaxActiveClusters, cached per
-// n and C). Inverse path 4 forces the largest C the block size allows.
+template <int TH, int RPL, bool RES>
+int launch3(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s, int c) {
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  QTX_TRY((configure3<TH, RPL, RES>(n, batch, c, &cfg, &attr, s)));
+  ProfScope prof(QTX_KERNEL_ZINV, 8.0 * (double)n * n * n * (double)batch, s);
+  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, zinv3_kernel<TH, RPL, RES>, n, batch, A, X, info, active, c));
+  return QTX_OK;
+}
+
+// Clusters of c CTAs of the column-split kernel that the GPU runs at once.
+int active_clusters(int n, int c) {
+  static thread_local std::vector<std::pair<int64_t, int>> cache;  // (n * 16 + c, clusters)
+  const int64_t key = (int64_t)n * 16 + c;
+  for (auto& e : cache)
+    if (e.first == key) return e.second;
+  cudaLaunchConfig_t cfg;
+  cudaLaunchAttribute attr;
+  int nc = 0;
+  cudaError_t e = cudaErrorUnknown;
+  if (n <= 128) {
+    if (configure3<512, 4, false>(n, 148, c, &cfg, &attr, nullptr) == QTX_OK)
+      e = cudaOccupancyMaxActiveClusters(&nc, zinv3_kernel<512, 4, false>, &cfg);
+  } else if (n <= 256) {
+    if (configure3<512, 8, false>(n, 148, c, &cfg, &attr, nullptr) == QTX_OK)
+      e = cudaOccupancyMaxActiveClusters(&nc, zinv3_kernel<512, 8, false>, &cfg);
+  } else {
+    if (configure3<512, 16, false>(n, 148, c, &cfg, &attr, nullptr) == QTX_OK)
+      e = cudaOccupancyMaxActiveClusters(&nc, zinv3_kernel<512, 16, false>, &cfg);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    nc = 0;
+  }
+  cache.emplace_back(key, nc);
+  return nc;
+}
+
+constexpr size_t kMaxSmem3 = 227 * 1024 - sizeof(GjPanelSmem<16>) - 64;  // beside the static shared memory
+bool fits_resident(int n) { return n <= 128 && Smem3::bytes(n, 1, true) <= kMaxSmem3; }
+
+// Column split of the n <= 512 kernel: the largest C in {1, 2, 4, 8} with
+// batch x C within the SM count, at least 32 columns per CTA, and all batch
+// clusters co-resident. Inverse path 4 forces the largest C the block size
+// allows; 2 is the least where one CTA's pivot rows and transform do not fit.
 int column_split(int n, int64_t batch) {
   const int path = inverse_path();
-  if ((path != 0 && path != 4) || n > 400) return 1;
+  int least = 1;
+  while (Smem3::bytes(n, least, false) > kMaxSmem3) least *= 2;
+  if (path != 0 && path != 4) return least;
   int cmax = 1;
   while (cmax < 8 && n / (2 * cmax) >= 32) cmax *= 2;
-  if (path == 4) return cmax;
+  if (path == 4) return cmax > least ? cmax : least;
   const int sms = num_sms();
-  int c = 1;
+  int c = least;
   while (c < cmax && batch * (2 * c) <= sms) c *= 2;
-  while (c > 1) {
-    static thread_local std::vector<std::pair<int64_t, int>> cache;  // (n * 16 + c, active clusters)
-    const int64_t key = (int64_t)n * 16 + c;
-    int active = -1;
-    for (auto& e : cache)
-      if (e.first == key) active = e.second;
-    if (active < 0) {
-      const size_t smem = Smem2<16>::bytes(n);
-      if (cudaFuncSetAttribute(zinv2_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) !=
-          cudaSuccess)
-        return 1;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = dim3((unsigned)(c * batch), 1, 1);
-      cfg.blockDim = dim3(T2, 1, 1);
-      cfg.dynamicSmemBytes = smem;
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = (unsigned)c;
-      attr[0].val.clusterDim.y = 1;
-      attr[0].val.clusterDim.z = 1;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      int nc = 0;
-      if (cudaOccupancyMaxActiveClusters(&nc, zinv2_kernel<16>, &cfg) != cudaSuccess) {
-        cudaGetLastError();
-        nc = 0;
-      }
-      active = nc;
-      cache.emplace_back(key, active);
-    }
-    if (active >= batch) return c;
-    c /= 2;
+  while (c > least && active_clusters(n, c) < batch) c /= 2;
+  return c;
+}
+
+int launch_split(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s) {
+  const int c = column_split(n, batch);
+  if (inverse_path() != 4 && fits_resident(n)) {
+    if (n <= 64) return launch3<256, 2, true>(n, batch, A, X, info, active, s, 1);
+    return launch3<512, 4, true>(n, batch, A, X, info, active, s, 1);
   }
-  return 1;
+  if (n <= 128) return launch3<512, 4, false>(n, batch, A, X, info, active, s, c);
+  if (n <= 256) return launch3<512, 8, false>(n, batch, A, X, info, active, s, c);
+  return launch3<512, 16, false>(n, batch, A, X, info, active, s, c);
 }
 
 }  // namespace
@@ -807,7 +1021,7 @@ int zinv(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active,
     return QTX_ERR_ARG;
   }
   if (zinv_prefers_cluster(n, batch)) return zinv_cluster(n, batch, A, X, info, active, s);
-  if (n <= 400) return launch2<16>(n, batch, A, X, info, active, s, column_split(n, batch));
+  if (n <= 512) return launch_split(n, batch, A, X, info, active, s);
   if (n <= 720) return launch2<8>(n, batch, A, X, info, active, s);
   if (n <= 1024) return launch<8>(n, batch, A, X, info, active, s);
   set_error("zinv: block sizes above 1024 are not supported");

@@ -7,10 +7,9 @@
 // rule (largest |Re| + |Im| at or below the diagonal, lowest row on ties) and
 // the same info convention (1-based column of the first zero pivot).
 //
-// Why: the one-CTA kernel streams the n x n matrix through HBM once per
-// 16-column panel (16 passes at n = 256) and takes ~1.7 ms per matrix; the
-// multi-CTA path pays three launches per panel. For batches below a few
-// times the number of clusters the device can hold, a cluster of
+// Why: the column-split kernel streams the n x n matrix through L2 or HBM once
+// per 16-column panel (16 passes at n = 256); the multi-CTA path pays three
+// launches per panel. While all clusters of a batch are resident, a cluster of
 // C = ceil(n / 32) CTAs (8 at n = 256) holds the matrix entirely in shared
 // memory -- 32 columns per CTA -- and runs every panel on chip:
 //
@@ -18,8 +17,7 @@
 //           3-D tensor map over (re/im doubles, rows, batch), 128-byte
 //           swizzle, no multicast) into four [rows][8 complex] chunks;
 //   panel:  the CTA owning the 16 columns of panel K factors them in place
-//           (pivot search, Smith reciprocal, elimination of every row), then
-//           arrives on the cluster barrier;
+//           (gj_panel.cuh), then arrives on the cluster barrier;
 //   update: every CTA reads the panel transform T = X[:, K] and the pivot
 //           rows from the owner's shared memory (DSMEM), applies the row
 //           interchanges to its own columns and updates them,
@@ -86,7 +84,7 @@ __device__ __forceinline__ int xoff(int npad, int r, int j) {
 struct ClusterSmem {
   // byte offsets inside the dynamic shared memory (base aligned to 1024)
   int npad;
-  size_t x, t, y, piv, colsrc, red_v, red_i, bar, total;
+  size_t x, t, y, piv, colsrc, bar, total;
   __host__ __device__ explicit ClusterSmem(int n) {
     npad = (n + 15) & ~15;
     x = 0;                                                  // 4 chunks [npad][8]
@@ -94,9 +92,7 @@ struct ClusterSmem {
     y = t + (size_t)2 * npad * 8 * sizeof(z64);             // [CNB][YS]
     piv = y + (size_t)CNB * YS * sizeof(z64);               // npad ints
     colsrc = piv + (size_t)npad * sizeof(int);              // npad ints
-    red_v = colsrc + (size_t)npad * sizeof(int);
-    red_i = red_v + (size_t)CWARPS * sizeof(double);
-    bar = (red_i + (size_t)CWARPS * sizeof(int) + 15) & ~(size_t)15;  // 2 mbarriers
+    bar = (colsrc + (size_t)npad * sizeof(int) + 15) & ~(size_t)15;  // 2 mbarriers
     total = bar + 16 + 1024;  // + alignment slack of the base
   }
 };
@@ -141,12 +137,9 @@ __global__ void __launch_bounds__(CT, 1)
   z64* Ys = reinterpret_cast<z64*>(base + L.y);
   int* pivrow = reinterpret_cast<int*>(base + L.piv);
   int* colsrc = reinterpret_cast<int*>(base + L.colsrc);
-  double* red_v = reinterpret_cast<double*>(base + L.red_v);
-  int* red_i = reinterpret_cast<int*>(base + L.red_i);
   uint64_t* lbar = reinterpret_cast<uint64_t*>(base + L.bar);  // the load of A
   uint64_t* tbar = lbar + 1;                                    // the panel transforms
   __shared__ int s_sing, s_first;
-  __shared__ z64 prow[CNB], rowk[CNB];
 
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int g = lane >> 2, tq = lane & 3;
@@ -198,10 +191,10 @@ __global__ void __launch_bounds__(CT, 1)
     const uint32_t tbytes = (uint32_t)(2 * chunk * sizeof(z64)) + CNB * sizeof(int);
 
     if (own) {
-      gj_factor_panel16(
-          n, k0, nbp, [&](int r, int c) { return Xs[xoff(npad, r, kl + c)]; },
-          [&](int r, int c, z64 v) { Xs[xoff(npad, r, kl + c)] = v; }, pivrow, prow, rowk, red_v, red_i,
-          &s_sing);
+      gj_factor_panel<CNB>(
+          n, k0, nbp, [=](int r, int c) { return Xs[xoff(npad, r, kl + c)]; },
+          [=](int r, int c, z64 v) { Xs[xoff(npad, r, kl + c)] = v; }, [](int, int) {},
+          [=](int k, int p) { pivrow[k] = p; }, &s_sing);
       // the panel's stores must be visible to the bulk copies below
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     } else if (tid == 0) {

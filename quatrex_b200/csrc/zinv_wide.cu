@@ -310,13 +310,13 @@ bool zinv_prefers_cluster(int n, int64_t batch) {
   if (n > 256) return false;
   if (g_inverse_path == 3) return true;
   if (g_inverse_path != 0) return false;
-  // A cluster per matrix (ceil(n / 32) CTAs, one per SM at n = 256) finishes
-  // one matrix 2.2x sooner than one CTA streaming it through HBM (0.59 vs
-  // 1.31 ms at n = 256), but holds C SMs for it, and the GPU co-schedules
-  // only about half of the SM count in clusters of 8: measured on B200, it
-  // wins while batch x C stays within half the SMs (n = 256: batch <= 9).
+  // A cluster per matrix (ceil(n / 32) CTAs) keeps it in shared memory but
+  // holds C SMs for it, and the GPU co-schedules only about half of the SM
+  // count in clusters of 8 (all of it in clusters of 4). Measured on B200
+  // against the column split: n = 128, batch 32 157 / 200 us; n = 64, batch 64
+  // 75 / 79 us; n = 256, batch 9 448 / 496 us but batch 18 886 / 629 us.
   const int c = (n + 31) / 32;
-  return batch * c * 2 <= (int64_t)num_sms();
+  return batch * c * (c <= 4 ? 1 : 2) <= (int64_t)num_sms();
 }
 
 bool zinv_prefers_wide(int n, int64_t batch) {
@@ -324,11 +324,11 @@ bool zinv_prefers_wide(int n, int64_t batch) {
   if (g_inverse_path == 2) return true;
   // One CTA per matrix leaves SMs idle when the batch is below the SM count;
   // the multi-CTA path pays n/NB launches and a pass over the matrix per
-  // panel. Up to n = 400 the column-split clusters of the one-CTA kernel
-  // (zinv.cu) use the idle SMs instead; above, the measured crossover on
-  // B200 (TFLOP/s of both paths against the batch) is batch 64 at n = 512.
+  // panel. Up to n = 512 the column-split clusters of zinv.cu use the idle SMs
+  // instead (n = 512, batch 21 / 42 / 74: 3.6 / 5.0 / 6.0 ms against 4.0 / 5.8
+  // / 8.3 ms); above, the measured crossover on B200 is half the SM count.
   const int sms = num_sms();
-  return n > 400 && batch * 2 <= sms;
+  return n > 512 && batch * 2 <= sms;
 }
 
 int zinv_ex(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, void* scratch,
