@@ -8,9 +8,9 @@
 // type (complex128 = double2 for the FP64 path, complex64 = float2 for the
 // mixed path); arithmetic is done in double either way. Transposed operands
 // are staged through a 32x32 shared-memory tile (one padding column) so
-// global loads and stores stay coalesced. Reductions use warp shuffles and
-// one shared-memory combine per CTA; one CTA reduces one stack entry, so
-// results are deterministic.
+// global loads and stores stay coalesced. Reductions cut an entry into fixed
+// bands of rows that the CTAs of a thread-block cluster sum (warp shuffles, one
+// shared-memory combine per band) and add in order: deterministic.
 #include <cooperative_groups.h>
 
 #include "common.cuh"
@@ -91,15 +91,24 @@ __global__ void __launch_bounds__(TILE* ROWS) combine_kernel(const CombineArgs a
   }
 }
 
-// out = 0.5 (X - X^H); density[b * ds + off + r] = Im X[r][r].
+// out_k = 0.5 (X_k - X_k^H) for `count` (1 or 2) stacks in one launch;
+// density[b * ds + off + r] = Im X_0[r][r].
+struct AntihermArgs {
+  MatRef X[2], out[2];
+};
 template <typename T>
 __global__ void __launch_bounds__(TILE* ROWS)
-    antiherm_kernel(int n, int64_t batch, MatRef X, MatRef out, double* dens, int64_t ds,
+    antiherm_kernel(int n, int64_t batch, int count, const AntihermArgs args, double* density, int64_t ds,
                     int64_t doff) {
   __shared__ z64 tile[TILE][TILE + 1];
   const int c0 = blockIdx.x * TILE, r0 = blockIdx.y * TILE;
   const int tx = threadIdx.x, ty = threadIdx.y;
-  for (int64_t b = blockIdx.z; b < batch; b += gridDim.z) {
+  for (int64_t z = blockIdx.z; z < batch * count; z += gridDim.z) {
+    const int k = z >= batch ? 1 : 0;
+    const int64_t b = z - k * batch;
+    const MatRef& X = args.X[k];
+    const MatRef& out = args.out[k];
+    double* dens = k == 0 ? density : nullptr;
     const T* x = at<const T>(X, b);
     __syncthreads();
 #pragma unroll
@@ -137,133 +146,172 @@ __device__ __forceinline__ V block_sum(V v, V* red) {
   return s;
 }
 
-// Tr(X Y) = sum_{r,c} X[r][c] Y[c][r], via 32x32 tiles (Y tile staged
-// transposed). A stack entry is reduced by the S CTAs of one thread-block
-// cluster (S = 1 for large batches): CTA s takes the row tiles s, s + S, ...
-// and the S partial sums are added in rank order by rank 0 through
-// distributed shared memory, so the result does not depend on timing.
-template <typename T>
-__global__ void __launch_bounds__(256) trace_kernel(int n, int64_t batch, MatRef X, MatRef Y, z64 coef,
-                                                    z64* res, int64_t rs, int64_t roff, int accumulate) {
-  __shared__ z64 tile[TILE][TILE + 1];
-  __shared__ double red[8];
-  __shared__ double part[2];
-  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  cg::cluster_group cluster = cg::this_cluster();
-  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
-  const int64_t b = blockIdx.x / S;  // uniform within a cluster
-  if (b < batch) {
-    const T* x = at<const T>(X, b);
-    const T* y = at<const T>(Y, b);
-    double sre = 0.0, sim = 0.0;
-    for (int r0 = rank * TILE; r0 < n; r0 += S * TILE)
-      for (int c0 = 0; c0 < n; c0 += TILE) {
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < TILE / ROWS; ++i) {
-          const int yr = c0 + ty + i * ROWS, yc = r0 + tx;
-          tile[ty + i * ROWS][tx] =
-              (yr < n && yc < n) ? ld2(y[(int64_t)yr * Y.ld + yc]) : make_double2(0, 0);
-        }
-        __syncthreads();
-#pragma unroll
-        for (int i = 0; i < TILE / ROWS; ++i) {
-          const int r = r0 + ty + i * ROWS, c = c0 + tx;
-          if (r < n && c < n) {
-            const z64 a = ld2(x[(int64_t)r * X.ld + c]);
-            const z64 w = tile[tx][ty + i * ROWS];  // Y[c][r]
-            sre += a.x * w.x - a.y * w.y;
-            sim += a.x * w.y + a.y * w.x;
-          }
-        }
-      }
-    sre = block_sum(sre, red);
-    sim = block_sum(sim, red);
-    if (threadIdx.x == 0) {
-      part[0] = sre;
-      part[1] = sim;
-    }
-  }
+// Reductions of one stack entry. An entry is cut into kChunks bands of rows,
+// each band is summed by one CTA (the S CTAs of the entry's thread-block
+// cluster take the bands rank, rank + S, ...), and rank 0 adds the bands in
+// order through distributed shared memory: the result depends neither on
+// timing nor on S. One CTA per entry leaves most SMs idle below 148 entries
+// and each thread with few loads in flight: the Sancho-Rubio measure of 128
+// entries of 256 x 256 took 205 us, against 41 us at the HBM rate.
+constexpr int kChunks = 8;
+constexpr int RT = 256;  // threads
+
+// Sum of the kChunks band partials (V values each) of this cluster's entry,
+// valid in rank 0's thread 0.
+template <int V>
+__device__ __forceinline__ void cluster_total(cg::cluster_group& cluster, double (&part)[kChunks][V], double (&tot)[V]) {
   cluster.sync();
-  if (b < batch && rank == 0 && threadIdx.x == 0) {
-    double tre = 0.0, tim = 0.0;
-    for (int q = 0; q < S; ++q) {
-      const double* pq = cluster.map_shared_rank(part, q);
-      tre += pq[0];
-      tim += pq[1];
+  if (cluster.block_rank() == 0 && threadIdx.x == 0) {
+    const int S = (int)cluster.num_blocks();
+#pragma unroll
+    for (int v = 0; v < V; ++v) tot[v] = 0.0;
+    for (int q = 0; q < kChunks; ++q) {
+      const double* pq = cluster.map_shared_rank(&part[q][0], q % S);
+#pragma unroll
+      for (int v = 0; v < V; ++v) tot[v] += pq[v];
     }
-    const z64 v = zmul(coef, make_double2(tre, tim));
-    z64* o = res + b * rs + roff;
-    *o = accumulate ? zadd(*o, v) : v;
   }
   cluster.sync();  // the partials stay readable until rank 0 has summed them
 }
 
-// delta[b] = sqrt(sum (|x| + |y|)^2) / 2.
-__global__ void __launch_bounds__(256) sr_delta_kernel(int n, int64_t batch, MatRef X, MatRef Y,
-                                                       double* delta, const int* active) {
-  __shared__ double red[8];
-  for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
-    if (active != nullptr && active[b] == 0) continue;
-    const z64* x = at<const z64>(X, b);
-    const z64* y = at<const z64>(Y, b);
-    double s = 0.0;
-    for (int64_t idx = threadIdx.x; idx < (int64_t)n * n; idx += blockDim.x) {
-      const int r = (int)(idx / n), c = (int)(idx % n);
-      const z64 a = x[(int64_t)r * X.ld + c];
-      const z64 w = y[(int64_t)r * Y.ld + c];
-      const double v = hypot(a.x, a.y) + hypot(w.x, w.y);
-      s += v * v;
-    }
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) delta[b] = 0.5 * sqrt(s);
-  }
-}
+struct TraceArgs {
+  int count;  // 1 or 2 products
+  MatRef X[2], Y[2];
+  z64 coef[2];
+};
 
-__global__ void __launch_bounds__(256) znorm_diff_kernel(int n, int64_t batch, MatRef X, MatRef Y,
-                                                         double* nd, double* nx, double* rel) {
-  __shared__ double red[8];
-  for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
-    const z64* x = at<const z64>(X, b);
-    const z64* y = at<const z64>(Y, b);
-    double sd = 0.0, sx = 0.0;
-    for (int64_t idx = threadIdx.x; idx < (int64_t)n * n; idx += blockDim.x) {
-      const int r = (int)(idx / n), c = (int)(idx % n);
-      const z64 a = x[(int64_t)r * X.ld + c];
-      const z64 w = y[(int64_t)r * Y.ld + c];
-      const double dr = a.x - w.x, di = a.y - w.y;
-      sd += dr * dr + di * di;
-      sx += a.x * a.x + a.y * a.y;
-    }
-    sd = block_sum(sd, red);
-    sx = block_sum(sx, red);
-    if (threadIdx.x == 0) {
-      if (nd != nullptr) nd[b] = sqrt(sd);
-      if (nx != nullptr) nx[b] = sqrt(sx);
-      if (rel != nullptr) rel[b] = sqrt(sd) / sqrt(sx);
-    }
-  }
-}
-
-// out[b] = Re sum conj(G) .* P  (= Re Tr(P G^H)).
+// res[b] = sum_k coef_k Tr(X_k Y_k), Tr(X Y) = sum_{r,c} X[r][c] Y[c][r] on
+// 32 x 32 tiles (the Y tile staged transposed).
 template <typename T>
-__global__ void __launch_bounds__(256) re_inner_kernel(int m, int n, int64_t batch, MatRef P, MatRef G,
-                                                       double* out) {
-  __shared__ double red[8];
-  for (int64_t b = blockIdx.x; b < batch; b += gridDim.x) {
-    const T* p = at<const T>(P, b);
-    const T* g = at<const T>(G, b);
-    double s = 0.0;
-    for (int64_t idx = threadIdx.x; idx < (int64_t)m * n; idx += blockDim.x) {
-      const int r = (int)(idx / n), c = (int)(idx % n);
-      const z64 a = ld2(p[(int64_t)r * P.ld + c]);
-      const z64 w = ld2(g[(int64_t)r * G.ld + c]);
-      s += a.x * w.x + a.y * w.y;
+__global__ void __launch_bounds__(RT) trace_kernel(int n, int64_t batch, const TraceArgs args, z64* res, int64_t rs,
+                                                   int64_t roff) {
+  __shared__ z64 tile[TILE][TILE + 1];
+  __shared__ double red[RT / 32];
+  __shared__ double part[kChunks][4];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  cg::cluster_group cluster = cg::this_cluster();
+  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int64_t b = blockIdx.x / S;  // uniform within a cluster
+  const int tiles = (n + TILE - 1) / TILE;
+  for (int q = rank; q < kChunks; q += S) {
+    double s[4] = {0.0, 0.0, 0.0, 0.0};
+    const int t0 = tiles * q / kChunks, t1 = tiles * (q + 1) / kChunks;
+    for (int k = 0; k < args.count && b < batch; ++k) {
+      const T* x = at<const T>(args.X[k], b);
+      const T* y = at<const T>(args.Y[k], b);
+      const int64_t ldx = args.X[k].ld, ldy = args.Y[k].ld;
+      double sre = 0.0, sim = 0.0;
+      for (int r0 = t0 * TILE; r0 < t1 * TILE; r0 += TILE)
+        for (int c0 = 0; c0 < n; c0 += TILE) {
+          z64 xv[TILE / ROWS], yv[TILE / ROWS];
+#pragma unroll
+          for (int i = 0; i < TILE / ROWS; ++i) {
+            const int yr = c0 + ty + i * ROWS, yc = r0 + tx;
+            yv[i] = (yr < n && yc < n) ? ld2(y[(int64_t)yr * ldy + yc]) : make_double2(0, 0);
+            const int r = r0 + ty + i * ROWS, c = c0 + tx;
+            xv[i] = (r < n && c < n) ? ld2(x[(int64_t)r * ldx + c]) : make_double2(0, 0);
+          }
+          __syncthreads();
+#pragma unroll
+          for (int i = 0; i < TILE / ROWS; ++i) tile[ty + i * ROWS][tx] = yv[i];
+          __syncthreads();
+#pragma unroll
+          for (int i = 0; i < TILE / ROWS; ++i) {
+            if (r0 + ty + i * ROWS < n && c0 + tx < n) {
+              const z64 w = tile[tx][ty + i * ROWS];  // Y[c][r]
+              sre += xv[i].x * w.x - xv[i].y * w.y;
+              sim += xv[i].x * w.y + xv[i].y * w.x;
+            }
+          }
+        }
+      s[2 * k] = sre;
+      s[2 * k + 1] = sim;
     }
-    s = block_sum(s, red);
-    if (threadIdx.x == 0) out[b] = s;
+#pragma unroll
+    for (int v = 0; v < 4; ++v) {
+      const double p = block_sum(s[v], red);
+      if (threadIdx.x == 0) part[q][v] = p;
+    }
+  }
+  double tot[4];
+  cluster_total<4>(cluster, part, tot);
+  if (b < batch && rank == 0 && threadIdx.x == 0) {
+    z64 v = zmul(args.coef[0], make_double2(tot[0], tot[1]));
+    if (args.count > 1) v = zadd(v, zmul(args.coef[1], make_double2(tot[2], tot[3])));
+    res[b * rs + roff] = v;
   }
 }
+
+// sum over the m x n elements of f(x, y) (V values), then done(b, totals).
+template <typename T, int V, class F, class Done>
+__global__ void __launch_bounds__(RT) reduce_kernel(int m, int n, int64_t batch, MatRef X, MatRef Y, F f, Done done,
+                                                    const int* active) {
+  __shared__ double red[RT / 32];
+  __shared__ double part[kChunks][V];
+  cg::cluster_group cluster = cg::this_cluster();
+  const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
+  const int64_t b = blockIdx.x / S;
+  if (b >= batch || (active != nullptr && active[b] == 0)) return;  // whole clusters
+  const T* x = at<const T>(X, b);
+  const T* y = at<const T>(Y, b);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  for (int q = rank; q < kChunks; q += S) {
+    double s[V];
+#pragma unroll
+    for (int v = 0; v < V; ++v) s[v] = 0.0;
+    const int r1 = (int)((int64_t)m * (q + 1) / kChunks);
+    for (int r = (int)((int64_t)m * q / kChunks) + warp; r < r1; r += RT / 32) {
+      const T* xr = x + (int64_t)r * X.ld;
+      const T* yr = y + (int64_t)r * Y.ld;
+#pragma unroll 4
+      for (int c = lane; c < n; c += 32) f(ld2(xr[c]), ld2(yr[c]), s);
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+      const double p = block_sum(s[v], red);
+      if (threadIdx.x == 0) part[q][v] = p;
+    }
+  }
+  double tot[V];
+  cluster_total<V>(cluster, part, tot);
+  if (rank == 0 && threadIdx.x == 0) done(b, tot);
+}
+
+// (|x| + |y|)^2; delta[b] = sqrt(sum) / 2.
+struct DeltaTerm {
+  __device__ __forceinline__ void operator()(z64 a, z64 w, double (&s)[1]) const {
+    const double v = sqrt(a.x * a.x + a.y * a.y) + sqrt(w.x * w.x + w.y * w.y);
+    s[0] += v * v;
+  }
+};
+struct DeltaDone {
+  double* delta;
+  __device__ void operator()(int64_t b, const double (&t)[1]) const { delta[b] = 0.5 * sqrt(t[0]); }
+};
+// |x - y|^2 and |x|^2.
+struct DiffTerm {
+  __device__ __forceinline__ void operator()(z64 a, z64 w, double (&s)[2]) const {
+    const double dr = a.x - w.x, di = a.y - w.y;
+    s[0] += dr * dr + di * di;
+    s[1] += a.x * a.x + a.y * a.y;
+  }
+};
+struct DiffDone {
+  double *nd, *nx, *rel;
+  __device__ void operator()(int64_t b, const double (&t)[2]) const {
+    if (nd != nullptr) nd[b] = sqrt(t[0]);
+    if (nx != nullptr) nx[b] = sqrt(t[1]);
+    if (rel != nullptr) rel[b] = sqrt(t[0]) / sqrt(t[1]);
+  }
+};
+// Re conj(y) x.
+struct InnerTerm {
+  __device__ __forceinline__ void operator()(z64 a, z64 w, double (&s)[1]) const { s[0] += a.x * w.x + a.y * w.y; }
+};
+struct InnerDone {
+  double* out;
+  __device__ void operator()(int64_t b, const double (&t)[1]) const { out[b] = t[0]; }
+};
 
 template <typename TI, typename TO>
 __global__ void convert_kernel(int m, int n, int64_t batch, MatRef in, MatRef out) {
@@ -277,7 +325,34 @@ __global__ void convert_kernel(int m, int n, int64_t batch, MatRef in, MatRef ou
 }
 
 unsigned grid_z(int64_t batch) { return (unsigned)(batch < 65535 ? batch : 65535); }
-unsigned grid_x(int64_t batch) { return (unsigned)(batch < 1048576 ? batch : 1048576); }
+
+// Cluster launch of one reduction: CTAs per entry, a power of two up to
+// kChunks while all CTAs of the batch are resident at once (8 per SM).
+cudaLaunchConfig_t cluster_config(int64_t batch, cudaLaunchAttribute* attr, cudaStream_t s) {
+  int S = 1;
+  while (S < kChunks && batch * S * 2 <= 8 * (int64_t)num_sms()) S *= 2;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(batch * S), 1, 1);
+  cfg.blockDim = dim3(RT, 1, 1);
+  cfg.stream = s;
+  attr->id = cudaLaunchAttributeClusterDimension;
+  attr->val.clusterDim.x = (unsigned)S;
+  attr->val.clusterDim.y = 1;
+  attr->val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cfg;
+}
+
+template <typename T, int V, class F, class Done>
+int reduce_t(int m, int n, int64_t batch, MatRef X, MatRef Y, F f, Done done, const int* active, cudaStream_t s) {
+  if (m <= 0 || n <= 0 || batch <= 0) return QTX_OK;
+  ProfScope prof(QTX_KERNEL_REDUCE, 2.0 * sizeof(T) * m * n * (double)batch, s);
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config(batch, &attr, s);
+  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, reduce_kernel<T, V, F, Done>, m, n, batch, X, Y, f, done, active));
+  return QTX_OK;
+}
 
 template <typename T>
 int combine_t(int m, int n, int64_t batch, MatRef out, const Addend* terms, int nterms,
@@ -306,48 +381,36 @@ int combine_t(int m, int n, int64_t batch, MatRef out, const Addend* terms, int 
 }
 
 template <typename T>
-int antiherm_t(int n, int64_t batch, MatRef X, MatRef out, double* density, int64_t dens_stride,
-               int64_t dens_off, cudaStream_t s) {
+int antiherm_t(int n, int64_t batch, int count, const MatRef* X, const MatRef* out, double* density,
+               int64_t dens_stride, int64_t dens_off, cudaStream_t s) {
   if (n <= 0 || batch <= 0) return QTX_OK;
-  dim3 grid((n + TILE - 1) / TILE, (n + TILE - 1) / TILE, grid_z(batch));
-  ProfScope prof(QTX_KERNEL_BLOCKOPS, 2.0 * sizeof(T) * n * n * (double)batch, s);
-  antiherm_kernel<T><<<grid, dim3(TILE, ROWS), 0, s>>>(n, batch, X, out, density, dens_stride, dens_off);
+  AntihermArgs args{};
+  for (int k = 0; k < count; ++k) {
+    args.X[k] = X[k];
+    args.out[k] = out[k];
+  }
+  dim3 grid((n + TILE - 1) / TILE, (n + TILE - 1) / TILE, grid_z(batch * count));
+  ProfScope prof(QTX_KERNEL_BLOCKOPS, 2.0 * sizeof(T) * n * n * (double)batch * count, s);
+  antiherm_kernel<T><<<grid, dim3(TILE, ROWS), 0, s>>>(n, batch, count, args, density, dens_stride, dens_off);
   QTX_CHECK_LAUNCH();
   return QTX_OK;
 }
 
 template <typename T>
-int trace_t(int n, int64_t batch, MatRef X, MatRef Y, z64 coef, z64* result, int64_t rstride,
-            int64_t roff, int accumulate, cudaStream_t s) {
-  if (n <= 0 || batch <= 0) return QTX_OK;
-  ProfScope prof(QTX_KERNEL_REDUCE, 2.0 * sizeof(T) * n * n * (double)batch, s);
-  // CTAs per stack entry: enough for two waves of the SMs, at most 8 (a
-  // portable cluster) and at most one per 32-row tile.
-  int S = 1;
-  while (S < 8 && (int64_t)S * 2 * batch <= 2 * 148 && S * TILE < n) S *= 2;
-  if ((int64_t)batch * S > 0x7fffffffll) S = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(batch * S), 1, 1);
-  cfg.blockDim = dim3(256, 1, 1);
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = S;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, trace_kernel<T>, n, batch, X, Y, coef, result, rstride, roff, accumulate));
-  return QTX_OK;
-}
-
-template <typename T>
-int re_inner_t(int m, int n, int64_t batch, MatRef P, MatRef G, double* out, cudaStream_t s) {
-  if (m <= 0 || n <= 0 || batch <= 0) return QTX_OK;
-  ProfScope prof(QTX_KERNEL_REDUCE, 2.0 * sizeof(T) * m * n * (double)batch, s);
-  re_inner_kernel<T><<<grid_x(batch), 256, 0, s>>>(m, n, batch, P, G, out);
-  QTX_CHECK_LAUNCH();
+int trace_t(int n, int64_t batch, int count, const MatRef* X, const MatRef* Y, const z64* coef, z64* result,
+            int64_t rstride, int64_t roff, cudaStream_t s) {
+  if (n <= 0 || batch <= 0 || count <= 0) return QTX_OK;
+  TraceArgs args{};
+  args.count = count;
+  for (int k = 0; k < count; ++k) {
+    args.X[k] = X[k];
+    args.Y[k] = Y[k];
+    args.coef[k] = coef[k];
+  }
+  ProfScope prof(QTX_KERNEL_REDUCE, 2.0 * sizeof(T) * n * n * (double)batch * count, s);
+  cudaLaunchAttribute attr;
+  const cudaLaunchConfig_t cfg = cluster_config(batch, &attr, s);
+  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, trace_kernel<T>, n, batch, args, result, rstride, roff));
   return QTX_OK;
 }
 
@@ -374,47 +437,35 @@ int ccombine(int m, int n, int64_t batch, MatRef out, const Addend* terms, int n
   return combine_t<float2>(m, n, batch, out, terms, nterms, active, s);
 }
 
-int zantiherm(int n, int64_t batch, MatRef X, MatRef out, double* density, int64_t dens_stride,
-              int64_t dens_off, cudaStream_t s) {
-  return antiherm_t<double2>(n, batch, X, out, density, dens_stride, dens_off, s);
+int zantiherm(int n, int64_t batch, int count, const MatRef* X, const MatRef* out, double* density,
+              int64_t dens_stride, int64_t dens_off, cudaStream_t s) {
+  return antiherm_t<double2>(n, batch, count, X, out, density, dens_stride, dens_off, s);
 }
-int cantiherm(int n, int64_t batch, MatRef X, MatRef out, double* density, int64_t dens_stride,
-              int64_t dens_off, cudaStream_t s) {
-  return antiherm_t<float2>(n, batch, X, out, density, dens_stride, dens_off, s);
-}
-
-int ztrace_prod(int n, int64_t batch, MatRef X, MatRef Y, z64 coef, z64* result, int64_t rstride,
-                int64_t roff, int accumulate, cudaStream_t s) {
-  return trace_t<double2>(n, batch, X, Y, coef, result, rstride, roff, accumulate, s);
-}
-int ctrace_prod(int n, int64_t batch, MatRef X, MatRef Y, z64 coef, z64* result, int64_t rstride,
-                int64_t roff, int accumulate, cudaStream_t s) {
-  return trace_t<float2>(n, batch, X, Y, coef, result, rstride, roff, accumulate, s);
+int cantiherm(int n, int64_t batch, int count, const MatRef* X, const MatRef* out, double* density,
+              int64_t dens_stride, int64_t dens_off, cudaStream_t s) {
+  return antiherm_t<float2>(n, batch, count, X, out, density, dens_stride, dens_off, s);
 }
 
-int sr_delta(int n, int64_t batch, MatRef X, MatRef Y, double* delta, const int* active,
-             cudaStream_t s) {
-  if (n <= 0 || batch <= 0) return QTX_OK;
-  ProfScope prof(QTX_KERNEL_REDUCE, 32.0 * n * n * (double)batch, s);
-  sr_delta_kernel<<<grid_x(batch), 256, 0, s>>>(n, batch, X, Y, delta, active);
-  QTX_CHECK_LAUNCH();
-  return QTX_OK;
+int ztrace_prod(int n, int64_t batch, int count, const MatRef* X, const MatRef* Y, const z64* coef, z64* result,
+                int64_t rstride, int64_t roff, cudaStream_t s) {
+  return trace_t<double2>(n, batch, count, X, Y, coef, result, rstride, roff, s);
+}
+int ctrace_prod(int n, int64_t batch, int count, const MatRef* X, const MatRef* Y, const z64* coef, z64* result,
+                int64_t rstride, int64_t roff, cudaStream_t s) {
+  return trace_t<float2>(n, batch, count, X, Y, coef, result, rstride, roff, s);
+}
+
+int sr_delta(int n, int64_t batch, MatRef X, MatRef Y, double* delta, const int* active, cudaStream_t s) {
+  return reduce_t<double2, 1>(n, n, batch, X, Y, DeltaTerm{}, DeltaDone{delta}, active, s);
 }
 
 int znorm_diff(int n, int64_t batch, MatRef X, MatRef Y, double* nrm_diff, double* nrm,
                double* rel, cudaStream_t s) {
-  if (n <= 0 || batch <= 0) return QTX_OK;
-  ProfScope prof(QTX_KERNEL_REDUCE, 32.0 * n * n * (double)batch, s);
-  znorm_diff_kernel<<<grid_x(batch), 256, 0, s>>>(n, batch, X, Y, nrm_diff, nrm, rel);
-  QTX_CHECK_LAUNCH();
-  return QTX_OK;
+  return reduce_t<double2, 2>(n, n, batch, X, Y, DiffTerm{}, DiffDone{nrm_diff, nrm, rel}, nullptr, s);
 }
 
 int zre_inner(int m, int n, int64_t batch, MatRef P, MatRef G, double* out, cudaStream_t s) {
-  return re_inner_t<double2>(m, n, batch, P, G, out, s);
-}
-int cre_inner(int m, int n, int64_t batch, MatRef P, MatRef G, double* out, cudaStream_t s) {
-  return re_inner_t<float2>(m, n, batch, P, G, out, s);
+  return reduce_t<double2, 1>(m, n, batch, P, G, InnerTerm{}, InnerDone{out}, nullptr, s);
 }
 
 int convert_c64_to_c128(int m, int n, int64_t batch, MatRef in, MatRef out, cudaStream_t s) {

@@ -116,6 +116,9 @@ struct GemmDesc {
 };
 
 int zgemm(const GemmDesc& d, cudaStream_t s);
+// Independent products (no output is an operand, addend or output of another);
+// consecutive ones of the same sizes and operations run in one launch.
+int zgemm_many(const GemmDesc* d, int count, cudaStream_t s);
 
 // The same GEMM emulated on the int8 tensor cores with `slices` digit planes
 // per operand (zgemm_oz.cu); `scratch` holds the planes of a batch chunk.
@@ -183,22 +186,23 @@ int zcombine(int m, int n, int64_t batch, MatRef out, const Addend* terms, int n
 int ccombine(int m, int n, int64_t batch, MatRef out, const Addend* terms, int nterms,
              const int* active, cudaStream_t s);
 
-// out = 0.5 (X - X^H); optional density[b, off + r] = Im X[r, r].
-int zantiherm(int n, int64_t batch, MatRef X, MatRef out, double* density, int64_t dens_stride,
-              int64_t dens_off, cudaStream_t s);
-int cantiherm(int n, int64_t batch, MatRef X, MatRef out, double* density, int64_t dens_stride,
-              int64_t dens_off, cudaStream_t s);
+// out_k = 0.5 (X_k - X_k^H), k < count (1 or 2), in one launch; optional
+// density[b, off + r] = Im X_0[r, r].
+int zantiherm(int n, int64_t batch, int count, const MatRef* X, const MatRef* out, double* density,
+              int64_t dens_stride, int64_t dens_off, cudaStream_t s);
+int cantiherm(int n, int64_t batch, int count, const MatRef* X, const MatRef* out, double* density,
+              int64_t dens_stride, int64_t dens_off, cudaStream_t s);
 
 // Element-type conversion of an m x n stack.
 int convert_c64_to_c128(int m, int n, int64_t batch, MatRef in, MatRef out, cudaStream_t s);
 int convert_c128_to_c64(int m, int n, int64_t batch, MatRef in, MatRef out, cudaStream_t s);
 
-// result[b * rstride + roff] (+)= sign * Tr(X_b Y_b)  (complex, n x n).
-int ztrace_prod(int n, int64_t batch, MatRef X, MatRef Y, z64 coef, z64* result, int64_t rstride,
-                int64_t roff, int accumulate, cudaStream_t s);
-
-int ctrace_prod(int n, int64_t batch, MatRef X, MatRef Y, z64 coef, z64* result, int64_t rstride,
-                int64_t roff, int accumulate, cudaStream_t s);
+// result[b * rstride + roff] = sum_k coef_k Tr(X_k,b Y_k,b), k < count (1 or 2;
+// complex, n x n).
+int ztrace_prod(int n, int64_t batch, int count, const MatRef* X, const MatRef* Y, const z64* coef, z64* result,
+                int64_t rstride, int64_t roff, cudaStream_t s);
+int ctrace_prod(int n, int64_t batch, int count, const MatRef* X, const MatRef* Y, const z64* coef, z64* result,
+                int64_t rstride, int64_t roff, cudaStream_t s);
 
 // delta[b] = || |X_b| + |Y_b| ||_F / 2   (Sancho-Rubio convergence measure).
 int sr_delta(int n, int64_t batch, MatRef X, MatRef Y, double* delta, const int* active,
@@ -211,7 +215,6 @@ int znorm_diff(int n, int64_t batch, MatRef X, MatRef Y, double* nrm_diff, doubl
 
 // T[b] = Re Tr(GamL G GamR G^H) given P = GamL G GamR: Re sum conj(G) .* P.
 int zre_inner(int m, int n, int64_t batch, MatRef P, MatRef G, double* out, cudaStream_t s);
-int cre_inner(int m, int n, int64_t batch, MatRef P, MatRef G, double* out, cudaStream_t s);
 
 // Launch profiler (profile.cu): RAII bracket of one kernel launch.
 // Scopes nest: only the outermost scope of a thread records, with `launches`

@@ -87,6 +87,13 @@ struct Gemm {
   int run(cudaStream_t s) { return zgemm(d, s); }
 };
 
+// Independent products, in as few launches as their sizes allow.
+int run_all(const std::vector<Gemm>& list, cudaStream_t s) {
+  std::vector<GemmDesc> d;
+  for (const Gemm& g : list) d.push_back(g.d);
+  return zgemm_many(d.data(), (int)d.size(), s);
+}
+
 int copy_block(int m, int n, int64_t batch, MatRef dst, MatRef src, cudaStream_t s) {
   if (dst.null()) return QTX_OK;
   Addend t = add(src, ONE);
@@ -147,13 +154,13 @@ int selected_inv_run(const BTRef& a, const MatRef* obc_r, const BTRef& x, int64_
   for (int i = N - 2; i >= 0; --i) {
     const int j = i + 1;
     MatRef T1 = shaped(tT, bs[i]);
-    QTX_TRY(Gemm(bs[j], bs[i], bs[j], batch, Gj, 0, a.lower[i], 0, T1).run(s));
-    MatRef xji = x.lower[i].null() ? shaped(tXji, bs[i]) : x.lower[i];
-    QTX_TRY(Gemm(bs[j], bs[i], bs[i], batch, T1, 0, g[i], 0, xji, MONE).run(s));
     MatRef U = shaped(tU, bs[j]);
-    QTX_TRY(Gemm(bs[i], bs[j], bs[i], batch, g[i], 0, a.upper[i], 0, U).run(s));
-    if (!x.upper[i].null())
-      QTX_TRY(Gemm(bs[i], bs[j], bs[j], batch, U, 0, Gj, 0, x.upper[i], MONE).run(s));
+    QTX_TRY(run_all({Gemm(bs[j], bs[i], bs[j], batch, Gj, 0, a.lower[i], 0, T1),
+                     Gemm(bs[i], bs[j], bs[i], batch, g[i], 0, a.upper[i], 0, U)}, s));
+    MatRef xji = x.lower[i].null() ? shaped(tXji, bs[i]) : x.lower[i];
+    std::vector<Gemm> off{Gemm(bs[j], bs[i], bs[i], batch, T1, 0, g[i], 0, xji, MONE)};
+    if (!x.upper[i].null()) off.push_back(Gemm(bs[i], bs[j], bs[j], batch, U, 0, Gj, 0, x.upper[i], MONE));
+    QTX_TRY(run_all(off, s));
     MatRef Gi = x.diag[i].null() ? shaped(tG[i & 1], bs[i]) : x.diag[i];
     QTX_TRY(Gemm(bs[i], bs[i], bs[j], batch, U, 0, xji, 0, Gi, MONE).plus(g[i], ONE).run(s));
     Gj = Gi;
@@ -177,13 +184,13 @@ struct Fp64 {
   static int combine(int m, int n, int64_t b, MatRef out, const Addend* t, int nt, cudaStream_t s) {
     return zcombine(m, n, b, out, t, nt, nullptr, s);
   }
-  static int antiherm(int n, int64_t b, MatRef X, MatRef out, double* d, int64_t ds, int64_t doff,
+  static int antiherm(int n, int64_t b, const MatRef* X, const MatRef* out, double* d, int64_t ds, int64_t doff,
                       cudaStream_t s) {
-    return zantiherm(n, b, X, out, d, ds, doff, s);
+    return zantiherm(n, b, 2, X, out, d, ds, doff, s);
   }
-  static int trace(int n, int64_t b, MatRef X, MatRef Y, z64 coef, z64* r, int64_t rs, int64_t ro,
-                   int acc, cudaStream_t s) {
-    return ztrace_prod(n, b, X, Y, coef, r, rs, ro, acc, s);
+  static int trace(int n, int64_t b, int count, const MatRef* X, const MatRef* Y, const z64* coef, z64* r,
+                   int64_t rs, int64_t ro, cudaStream_t s) {
+    return ztrace_prod(n, b, count, X, Y, coef, r, rs, ro, s);
   }
   static int inv(int n, int64_t b, MatRef X, int* info, MatRef, void* scr, size_t scr_bytes, cudaStream_t s) {
     return zinv_ex(n, b, X, X, info, nullptr, scr, scr_bytes, s);
@@ -243,6 +250,11 @@ struct MixedGemm {
   }
 };
 
+int run_all(std::vector<MixedGemm> list, cudaStream_t s) {
+  for (MixedGemm& g : list) QTX_TRY(g.run(s));
+  return QTX_OK;
+}
+
 struct Mixed {
   static constexpr size_t E = sizeof(c32);
   static constexpr bool kInvTmp = true;
@@ -250,13 +262,13 @@ struct Mixed {
   static int combine(int m, int n, int64_t b, MatRef out, const Addend* t, int nt, cudaStream_t s) {
     return ccombine(m, n, b, out, t, nt, nullptr, s);
   }
-  static int antiherm(int n, int64_t b, MatRef X, MatRef out, double* d, int64_t ds, int64_t doff,
+  static int antiherm(int n, int64_t b, const MatRef* X, const MatRef* out, double* d, int64_t ds, int64_t doff,
                       cudaStream_t s) {
-    return cantiherm(n, b, X, out, d, ds, doff, s);
+    return cantiherm(n, b, 2, X, out, d, ds, doff, s);
   }
-  static int trace(int n, int64_t b, MatRef X, MatRef Y, z64 coef, z64* r, int64_t rs, int64_t ro,
-                   int acc, cudaStream_t s) {
-    return ctrace_prod(n, b, X, Y, coef, r, rs, ro, acc, s);
+  static int trace(int n, int64_t b, int count, const MatRef* X, const MatRef* Y, const z64* coef, z64* r,
+                   int64_t rs, int64_t ro, cudaStream_t s) {
+    return ctrace_prod(n, b, count, X, Y, coef, r, rs, ro, s);
   }
   // The Schur complement is inverted in FP64: upcast, Gauss-Jordan, round back.
   static int inv(int n, int64_t b, MatRef X, int* info, MatRef tmp, void* scr, size_t scr_bytes,
@@ -322,7 +334,11 @@ int solve_impl(const SolveIO& io, int64_t batch, int* info, Workspace& ws, cudaS
       st[x].resize(N);
       for (int i = 0; i < N; ++i) st[x][i] = ws.mat(bs[i], bs[i], batch, Prec::E);
     }
-  enum { P_, P2_, M_, T_, Q_, T2_, U_, V_, W_, Z_, R1_, TT_, T1X_, T2X_, Y_, XIJ_, GA_, GB_, CA_, CB_, NT_ };
+  // Temporaries; those of the forward sweep are free again in the backward
+  // one. A pair (x = 0, 1) holds the lesser and the greater product.
+  enum { GA_, GB_, CA_, CB_, P_, P2_, Q_, T_ = Q_ + 2, M_ = T_ + 2, T2_ = M_ + 2, NF_ = T2_ + 2,
+         U_ = P_, V_, Z_, R1_, Y_ = R1_ + 2, T1_ = Y_ + 2, TB_ = T1_ + 2, XIJ_ = TB_ + 2, NT_ = XIJ_ + 2 };
+  static_assert(NF_ <= NT_, "forward temporaries");
   MatRef tmp[NT_];
   for (int k = 0; k < NT_; ++k) tmp[k] = ws.mat(bm, bm, batch, Prec::E);
   MatRef inv_tmp = Prec::kInvTmp ? ws.mat(bm, bm, batch, sizeof(z64)) : MatRef{};
@@ -354,14 +370,16 @@ int solve_impl(const SolveIO& io, int64_t batch, int* info, Workspace& ws, cudaS
     Addend t[2] = {add(a.diag[0], ONE), add(obc(io.obc_r, 0), MONE)};
     QTX_TRY(Prec::combine(bs[0], bs[0], batch, gR[0], t, 2, s));
     QTX_TRY(Prec::inv(bs[0], batch, gR[0], info, inv_tmp, inv_scr, inv_scr_bytes, s));
+    std::vector<Gemm> l1, l2;
     for (int x = 0; x < 2; ++x) {
-      MatRef M = shaped(tmp[M_], bs[0]);
+      MatRef M = shaped(tmp[M_ + x], bs[0]), T2 = shaped(tmp[T2_ + x], bs[0]);
       Addend u[2] = {add(sdiag(x, 0), ONE), add(obc(obx[x], 0), ONE)};
       QTX_TRY(Prec::combine(bs[0], bs[0], batch, M, u, 2, s));
-      MatRef T2 = shaped(tmp[T2_], bs[0]);
-      QTX_TRY(Gemm(bs[0], bs[0], bs[0], batch, gR[0], 0, M, 0, T2).run(s));
-      QTX_TRY(Gemm(bs[0], bs[0], bs[0], batch, T2, 0, gR[0], 1, gX[x][0]).run(s));
+      l1.push_back(Gemm(bs[0], bs[0], bs[0], batch, gR[0], 0, M, 0, T2));
+      l2.push_back(Gemm(bs[0], bs[0], bs[0], batch, T2, 0, gR[0], 1, gX[x][0]));
     }
+    QTX_TRY(run_all(l1, s));
+    QTX_TRY(run_all(l2, s));
   }
   // Forward sweep (rgf.py:241-302). The retarded chain runs on the helper
   // stream `sr`; the lesser/greater products of block j wait for the inverse
@@ -394,44 +412,47 @@ int solve_impl(const SolveIO& io, int64_t batch, int* info, Workspace& ws, cudaS
       QTX_CHECK_CUDA(cudaEventRecord(ss->inv, sr));
       QTX_CHECK_CUDA(cudaStreamWaitEvent(s, ss->inv, 0));
     }
+    std::vector<Gemm> l1, l2, l3, l4;
     for (int x = 0; x < 2; ++x) {
-      MatRef Q{};
+      MatRef Q{}, T = shaped(tmp[T_ + x], bs[i]), M = shaped(tmp[M_ + x], bs[j]), T2 = shaped(tmp[T2_ + x], bs[j]);
       if (!supper(x, i).null()) {
-        Q = shaped(tmp[Q_], bs[j]);
-        QTX_TRY(Gemm(bs[j], bs[j], bs[i], batch, P, 0, supper(x, i), 0, Q).run(s));
+        Q = shaped(tmp[Q_ + x], bs[j]);
+        l1.push_back(Gemm(bs[j], bs[j], bs[i], batch, P, 0, supper(x, i), 0, Q));
       }
-      MatRef T = shaped(tmp[T_], bs[i]);
-      QTX_TRY(Gemm(bs[j], bs[i], bs[i], batch, a.lower[i], 0, gX[x][i], 0, T).run(s));
-      MatRef M = shaped(tmp[M_], bs[j]);
+      l1.push_back(Gemm(bs[j], bs[i], bs[i], batch, a.lower[i], 0, gX[x][i], 0, T));
       if (want_current) {
         // Sigma-tilde (rgf.py:392-402) kept for the current; M = it + Sigma_jj.
-        QTX_TRY(Gemm(bs[j], bs[j], bs[i], batch, T, 0, a.lower[i], 1, st[x][j])
-                    .plus(Q, ONE, 1)
-                    .plus(Q, MONE)
-                    .second(M, ONE)
-                    .plus3(sdiag(x, j), ONE)
-                    .plus3(obc(obx[x], j), ONE)
-                    .run(s));
+        l2.push_back(Gemm(bs[j], bs[j], bs[i], batch, T, 0, a.lower[i], 1, st[x][j])
+                         .plus(Q, ONE, 1)
+                         .plus(Q, MONE)
+                         .second(M, ONE)
+                         .plus3(sdiag(x, j), ONE)
+                         .plus3(obc(obx[x], j), ONE));
       } else {
-        QTX_TRY(Gemm(bs[j], bs[j], bs[i], batch, T, 0, a.lower[i], 1, M)
-                    .plus(Q, ONE, 1)
-                    .plus(Q, MONE)
-                    .plus(sdiag(x, j), ONE)
-                    .plus(obc(obx[x], j), ONE)
-                    .run(s));
+        l2.push_back(Gemm(bs[j], bs[j], bs[i], batch, T, 0, a.lower[i], 1, M)
+                         .plus(Q, ONE, 1)
+                         .plus(Q, MONE)
+                         .plus(sdiag(x, j), ONE)
+                         .plus(obc(obx[x], j), ONE));
       }
-      MatRef T2 = shaped(tmp[T2_], bs[j]);
-      QTX_TRY(Gemm(bs[j], bs[j], bs[j], batch, gR[j], 0, M, 0, T2).run(s));
-      QTX_TRY(Gemm(bs[j], bs[j], bs[j], batch, T2, 0, gR[j], 1, gX[x][j]).run(s));
+      l3.push_back(Gemm(bs[j], bs[j], bs[j], batch, gR[j], 0, M, 0, T2));
+      l4.push_back(Gemm(bs[j], bs[j], bs[j], batch, T2, 0, gR[j], 1, gX[x][j]));
     }
+    if (l1.size() == 4) std::swap(l1[1], l1[2]);  // the pairs of one shape side by side
+    QTX_TRY(run_all(l1, s));
+    QTX_TRY(run_all(l2, s));
+    QTX_TRY(run_all(l3, s));
+    QTX_TRY(run_all(l4, s));
     if (use_side) QTX_CHECK_CUDA(cudaEventRecord(ss->xdone[j & 1], s));
   }
   // (The caller's stream has waited for the last inverse: every helper-stream
   // launch is ordered before what follows.)
   // Last diagonal blocks (rgf.py:305-312).
-  for (int x = 0; x < 2; ++x)
-    QTX_TRY(Prec::antiherm(bs[N - 1], batch, gX[x][N - 1], odiag(x, N - 1),
-                      x == 0 ? io.density : nullptr, dens_stride, offs[N - 1], s));
+  auto antiherm = [&](int i) {
+    const MatRef in[2] = {gX[0][i], gX[1][i]}, res[2] = {odiag(0, i), odiag(1, i)};
+    return Prec::antiherm(bs[i], batch, in, res, io.density, dens_stride, offs[i], s);
+  };
+  QTX_TRY(antiherm(N - 1));
   if (io.xr.n) QTX_TRY(copy_block_t<Prec>(bs[N - 1], bs[N - 1], batch, io.xr.diag[N - 1], gR[N - 1], s));
 
   // Backward sweep (rgf.py:315-412).
@@ -440,65 +461,64 @@ int solve_impl(const SolveIO& io, int64_t batch, int* info, Workspace& ws, cudaS
   const bool want_g0n = !io.g0n.null();
   for (int i = N - 2; i >= 0; --i) {
     const int j = i + 1;
-    MatRef U = shaped(tmp[U_], bs[j]);   // xr_ii a_ij
-    MatRef V = shaped(tmp[V_], bs[i]);   // xr_jj a_ji
-    MatRef W = shaped(tmp[W_], bs[j]);   // xr_ii a_ij xr_jj
-    MatRef Z = shaped(tmp[Z_], bs[i]);   // xr_ii a_ij xr_jj a_ji
-    QTX_TRY(Gemm(bs[i], bs[j], bs[i], batch, gR[i], 0, a.upper[i], 0, U).run(s));
-    QTX_TRY(Gemm(bs[j], bs[i], bs[j], batch, GRj, 0, a.lower[i], 0, V).run(s));
-    QTX_TRY(Gemm(bs[i], bs[j], bs[j], batch, U, 0, GRj, 0, W).run(s));
-    QTX_TRY(Gemm(bs[i], bs[i], bs[j], batch, U, 0, V, 0, Z).run(s));
+    MatRef U = shaped(tmp[U_], bs[j]);  // xr_ii a_ij
+    MatRef V = shaped(tmp[V_], bs[i]);  // xr_jj a_ji
+    MatRef Z = shaped(tmp[Z_], bs[i]);  // xr_ii a_ij xr_jj a_ji
+    // xr_ii <- xr_ii + xr_ii a_ij xr_jj a_ji xr_ii  (rgf.py:410).
+    MatRef Gi = (io.xr.n && !io.xr.diag[i].null()) ? io.xr.diag[i] : shaped(tmp[(i & 1) ? GA_ : GB_], bs[i]);
+    // Levels of independent products. With Y = xr_ii sigma_ij xr_jj^H the
+    // reference's xr_ii sigma_ij (xr_ii a_ij xr_jj)^H (rgf.py:346-349) is
+    // Y U^H, which needs no product xr_ii a_ij xr_jj.
+    std::vector<Gemm> l1, l2, ly, l3, l4, l5;
+    l1.push_back(Gemm(bs[i], bs[j], bs[i], batch, gR[i], 0, a.upper[i], 0, U));
+    l2.push_back(Gemm(bs[i], bs[i], bs[j], batch, U, 0, V, 0, Z));
+    l4.push_back(Gemm(bs[i], bs[i], bs[i], batch, Z, 0, gR[i], 0, Gi).plus(gR[i], ONE));
     for (int x = 0; x < 2; ++x) {
       const MatRef sx = supper(x, i);
-      MatRef R1{}, TT{};
+      MatRef Y{};
+      MatRef t1 = shaped(tmp[T1_ + x], bs[i]), t2 = shaped(tmp[TB_ + x], bs[j]);
       if (!sx.null()) {
-        R1 = shaped(tmp[R1_], bs[j]);
-        TT = shaped(tmp[TT_], bs[i]);
-        QTX_TRY(Gemm(bs[i], bs[j], bs[i], batch, gR[i], 0, sx, 0, R1).run(s));
-        QTX_TRY(Gemm(bs[i], bs[i], bs[j], batch, R1, 0, W, 1, TT).run(s));
+        MatRef R1 = shaped(tmp[R1_ + x], bs[j]);
+        Y = shaped(tmp[Y_ + x], bs[j]);
+        l1.push_back(Gemm(bs[i], bs[j], bs[i], batch, gR[i], 0, sx, 0, R1));
+        ly.push_back(Gemm(bs[i], bs[j], bs[j], batch, R1, 0, GRj, 1, Y));
+        l3.push_back(Gemm(bs[i], bs[i], bs[j], batch, Y, 0, U, 1, t1));
       }
-      MatRef t1 = shaped(tmp[T1X_], bs[i]);
-      QTX_TRY(Gemm(bs[i], bs[i], bs[i], batch, Z, 0, gX[x][i], 0, t1).plus(TT, MONE).run(s));
-      MatRef t2 = shaped(tmp[T2X_], bs[j]);
-      QTX_TRY(Gemm(bs[i], bs[j], bs[j], batch, U, 0, gX[x][j], 0, t2).run(s));
-      MatRef xij = oupper(x, i).null() ? shaped(tmp[XIJ_], bs[j]) : oupper(x, i);
+      l2.push_back(Gemm(bs[i], bs[j], bs[j], batch, U, 0, gX[x][j], 0, t2));
+      MatRef xij = oupper(x, i).null() ? shaped(tmp[XIJ_ + x], bs[j]) : oupper(x, i);
       MatRef xji = io.symmetric ? MatRef{} : olower(x, i);
-      if (!sx.null()) {
-        MatRef Y = shaped(tmp[Y_], bs[j]);
-        QTX_TRY(Gemm(bs[i], bs[j], bs[j], batch, R1, 0, GRj, 1, Y).plus(t2, MONE).run(s));
-        QTX_TRY(Gemm(bs[i], bs[j], bs[i], batch, gX[x][i], 0, V, 1, xij, MONE)
-                    .plus(Y, ONE)
-                    .store_h(xji, MONE)
-                    .run(s));
-      } else {
-        QTX_TRY(Gemm(bs[i], bs[j], bs[i], batch, gX[x][i], 0, V, 1, xij, MONE)
-                    .plus(t2, MONE)
-                    .store_h(xji, MONE)
-                    .run(s));
-      }
+      l3.push_back(Gemm(bs[i], bs[j], bs[i], batch, gX[x][i], 0, V, 1, xij, MONE)
+                       .plus(Y, ONE)
+                       .plus(t2, MONE)
+                       .store_h(xji, MONE));
+      l4.push_back(Gemm(bs[i], bs[i], bs[i], batch, Z, 0, gX[x][i], 0, t1).plus(Y.null() ? MatRef{} : t1, MONE));
       // X_ii = x_ii + temp_2x a_ij^H xr_ii^H + temp_1x - temp_1x^H (in place).
-      QTX_TRY(Gemm(bs[i], bs[i], bs[j], batch, t2, 0, U, 1, gX[x][i])
-                  .plus(gX[x][i], ONE)
-                  .plus(t1, ONE)
-                  .plus(t1, MONE, 1)
-                  .run(s));
-      QTX_TRY(Prec::antiherm(bs[i], batch, gX[x][i], odiag(x, i), x == 0 ? io.density : nullptr,
-                        dens_stride, offs[i], s));
+      l5.push_back(Gemm(bs[i], bs[i], bs[j], batch, t2, 0, U, 1, gX[x][i])
+                       .plus(gX[x][i], ONE)
+                       .plus(t1, ONE)
+                       .plus(t1, MONE, 1));
     }
-    if (want_current) {
-      // I_j = Tr(Sigma~^>_j X^<_jj - X^>_jj Sigma~^<_j)  (rgf.py:403-408).
-      QTX_TRY(Prec::trace(bs[j], batch, st[1][j], gX[0][j], ONE, io.current, cur_stride, j, 0, s));
-      QTX_TRY(Prec::trace(bs[j], batch, gX[1][j], st[0][j], MONE, io.current, cur_stride, j, 1, s));
-    }
+    l1.push_back(Gemm(bs[j], bs[i], bs[j], batch, GRj, 0, a.lower[i], 0, V));
     if (want_g0n) {
       MatRef nc = shaped(tmp[(i & 1) ? CA_ : CB_], bs[N - 1]);
       if (i == 0) nc = io.g0n;
-      QTX_TRY(Gemm(bs[i], bs[N - 1], bs[j], batch, U, 0, col, 0, nc, MONE).run(s));
+      l2.push_back(Gemm(bs[i], bs[N - 1], bs[j], batch, U, 0, col, 0, nc, MONE));
       col = nc;
     }
-    // xr_ii <- xr_ii + xr_ii a_ij xr_jj a_ji xr_ii  (rgf.py:410).
-    MatRef Gi = (io.xr.n && !io.xr.diag[i].null()) ? io.xr.diag[i] : shaped(tmp[(i & 1) ? GA_ : GB_], bs[i]);
-    QTX_TRY(Gemm(bs[i], bs[i], bs[i], batch, Z, 0, gR[i], 0, Gi).plus(gR[i], ONE).run(s));
+    if (l3.size() == 4) std::swap(l3[1], l3[2]);  // the pairs of one shape side by side
+    QTX_TRY(run_all(l1, s));
+    QTX_TRY(run_all(l2, s));
+    QTX_TRY(run_all(ly, s));
+    QTX_TRY(run_all(l3, s));
+    QTX_TRY(run_all(l4, s));
+    QTX_TRY(run_all(l5, s));
+    QTX_TRY(antiherm(i));
+    if (want_current) {
+      // I_j = Tr(Sigma~^>_j X^<_jj - X^>_jj Sigma~^<_j)  (rgf.py:403-408).
+      const MatRef tx[2] = {st[1][j], gX[1][j]}, ty[2] = {gX[0][j], st[0][j]};
+      const z64 tc[2] = {ONE, MONE};
+      QTX_TRY(Prec::trace(bs[j], batch, 2, tx, ty, tc, io.current, cur_stride, j, s));
+    }
     GRj = Gi;
   }
   if (want_g0n && N == 1) QTX_TRY(copy_block_t<Prec>(bs[0], bs[0], batch, io.g0n, gR[0], s));
@@ -508,15 +528,24 @@ int solve_impl(const SolveIO& io, int64_t batch, int* info, Workspace& ws, cudaS
     const MatRef ln = obc(io.obc_l, N - 1), gn = obc(io.obc_g, N - 1);
     // Slots 0 and N start from the caller's zero initialisation; a missing
     // OBC block contributes nothing.
-    if (!g0.null())
-      QTX_TRY(Prec::trace(bs[0], batch, g0, gX[0][0], ONE, io.current, cur_stride, 0, 0, s));
-    if (!l0.null())
-      QTX_TRY(Prec::trace(bs[0], batch, gX[1][0], l0, MONE, io.current, cur_stride, 0, g0.null() ? 0 : 1, s));
-    if (!gn.null())
-      QTX_TRY(Prec::trace(bs[N - 1], batch, gn, gX[0][N - 1], MONE, io.current, cur_stride, N, 0, s));
-    if (!ln.null())
-      QTX_TRY(Prec::trace(bs[N - 1], batch, gX[1][N - 1], ln, ONE, io.current, cur_stride, N,
-                          gn.null() ? 0 : 1, s));
+    auto boundary = [&](int i, int slot, const MatRef& ol, const MatRef& og, z64 sign) {
+      MatRef tx[2], ty[2];
+      z64 tc[2];
+      int n = 0;
+      if (!og.null()) {
+        tx[n] = og;
+        ty[n] = gX[0][i];
+        tc[n++] = sign;
+      }
+      if (!ol.null()) {
+        tx[n] = gX[1][i];
+        ty[n] = ol;
+        tc[n++] = make_double2(-sign.x, 0.0);
+      }
+      return Prec::trace(bs[i], batch, n, tx, ty, tc, io.current, cur_stride, slot, s);
+    };
+    QTX_TRY(boundary(0, 0, l0, g0, ONE));
+    QTX_TRY(boundary(N - 1, N, ln, gn, MONE));
   }
   return QTX_OK;
 }

@@ -159,6 +159,30 @@ int sr_load(int n, int64_t batch, int64_t off, const SRState& st, MatRef aii, Ma
   return QTX_OK;
 }
 
+// One decimation step from alpha[cur], beta[cur] to alpha[1 - cur],
+// beta[1 - cur], and its convergence measure. The products that do not need
+// one another share a launch.
+int sr_step(int n, int64_t batch, const SRState& st, int cur, int* info, const int* mask, cudaStream_t s) {
+  const int nx = cur ^ 1;
+  QTX_TRY(zinv_ex(n, batch, st.eps, st.inv_e, info, mask, st.scr, st.scr_bytes, s));
+  const GemmDesc left[2] = {G(n, n, n, batch, st.alpha[cur], st.inv_e, st.aI).mask(mask).d,
+                            G(n, n, n, batch, st.beta[cur], st.inv_e, st.bI).mask(mask).d};
+  QTX_TRY(zgemm_many(left, 2, s));
+  // t1 = alpha inv beta;  eps_s <- eps_s - t1.
+  const GemmDesc next[3] = {
+      G(n, n, n, batch, st.aI, st.beta[cur], st.t1).second(st.eps_s, MONE).plus3(st.eps_s, ONE).mask(mask).d,
+      G(n, n, n, batch, st.aI, st.alpha[cur], st.alpha[nx]).mask(mask).d,
+      G(n, n, n, batch, st.bI, st.beta[cur], st.beta[nx]).mask(mask).d};
+  QTX_TRY(zgemm_many(next, 3, s));
+  // eps <- eps - t1 - beta inv alpha.
+  QTX_TRY(G(n, n, n, batch, st.bI, st.alpha[cur], st.eps, MONE)
+              .plus(st.eps, ONE)
+              .plus(st.t1, MONE)
+              .mask(mask)
+              .run(s));
+  return sr_delta(n, batch, st.alpha[nx], st.beta[nx], st.delta, mask, s);
+}
+
 // The decimation loop on the whole state; eps_s holds the result.
 int sr_iterate(int n, int64_t batch, const SRState& st, int max_iterations, double tol,
                int per_energy, int* iterations, int* converged, int* info, cudaStream_t s) {
@@ -170,24 +194,7 @@ int sr_iterate(int n, int64_t batch, const SRState& st, int max_iterations, doub
   const int* mask = per_energy ? st.active : nullptr;
   while (it < max_iterations && !done) {
     const int nx = cur ^ 1;
-    QTX_TRY(zinv_ex(n, batch, st.eps, st.inv_e, info, mask, st.scr, st.scr_bytes, s));
-    QTX_TRY(G(n, n, n, batch, st.alpha[cur], st.inv_e, st.aI).mask(mask).run(s));
-    QTX_TRY(G(n, n, n, batch, st.beta[cur], st.inv_e, st.bI).mask(mask).run(s));
-    // t1 = alpha inv beta;  eps_s <- eps_s - t1.
-    QTX_TRY(G(n, n, n, batch, st.aI, st.beta[cur], st.t1)
-                .second(st.eps_s, MONE)
-                .plus3(st.eps_s, ONE)
-                .mask(mask)
-                .run(s));
-    // eps <- eps - t1 - beta inv alpha.
-    QTX_TRY(G(n, n, n, batch, st.bI, st.alpha[cur], st.eps, MONE)
-                .plus(st.eps, ONE)
-                .plus(st.t1, MONE)
-                .mask(mask)
-                .run(s));
-    QTX_TRY(G(n, n, n, batch, st.aI, st.alpha[cur], st.alpha[nx]).mask(mask).run(s));
-    QTX_TRY(G(n, n, n, batch, st.bI, st.beta[cur], st.beta[nx]).mask(mask).run(s));
-    QTX_TRY(sr_delta(n, batch, st.alpha[nx], st.beta[nx], st.delta, mask, s));
+    QTX_TRY(sr_step(n, batch, st, cur, info, mask, s));
     ++it;
     QTX_CHECK_CUDA(cudaMemcpyAsync(hdelta.data(), st.delta, sizeof(double) * batch,
                                    cudaMemcpyDeviceToHost, s));
@@ -287,22 +294,7 @@ int sr_iterate_async(int n, int64_t batch, const SRState& st, int max_iterations
   const int* mask = st.active;
   for (int it = 0; it < max_iterations; ++it) {
     const int nx = cur ^ 1;
-    QTX_TRY(zinv_ex(n, batch, st.eps, st.inv_e, info, mask, st.scr, st.scr_bytes, s));
-    QTX_TRY(G(n, n, n, batch, st.alpha[cur], st.inv_e, st.aI).mask(mask).run(s));
-    QTX_TRY(G(n, n, n, batch, st.beta[cur], st.inv_e, st.bI).mask(mask).run(s));
-    QTX_TRY(G(n, n, n, batch, st.aI, st.beta[cur], st.t1)
-                .second(st.eps_s, MONE)
-                .plus3(st.eps_s, ONE)
-                .mask(mask)
-                .run(s));
-    QTX_TRY(G(n, n, n, batch, st.bI, st.alpha[cur], st.eps, MONE)
-                .plus(st.eps, ONE)
-                .plus(st.t1, MONE)
-                .mask(mask)
-                .run(s));
-    QTX_TRY(G(n, n, n, batch, st.aI, st.alpha[cur], st.alpha[nx]).mask(mask).run(s));
-    QTX_TRY(G(n, n, n, batch, st.bI, st.beta[cur], st.beta[nx]).mask(mask).run(s));
-    QTX_TRY(sr_delta(n, batch, st.alpha[nx], st.beta[nx], st.delta, mask, s));
+    QTX_TRY(sr_step(n, batch, st, cur, info, mask, s));
     {
       ProfScope prof(QTX_KERNEL_REDUCE, 12.0 * (double)batch, s);
       sr_update_kernel<<<1, 256, 0, s>>>(batch, st.delta, st.active, tol, per_energy, d_iters,

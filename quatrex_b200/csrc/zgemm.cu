@@ -380,8 +380,16 @@ bool aligned16(const MatRef& m) { return (reinterpret_cast<uintptr_t>(m.p) & 15u
 
 }  // namespace
 
-int zgemm(const GemmDesc& d, cudaStream_t s) {
-  if (d.M <= 0 || d.N <= 0 || d.batch <= 0) return QTX_OK;
+namespace {
+
+// Checks one product and brings it into the form the kernel takes (zero
+// operands and addends dropped). *skip: nothing to do.
+int normalize(const GemmDesc& d, GemmDesc* out, bool* skip) {
+  *skip = false;
+  if (d.M <= 0 || d.N <= 0 || d.batch <= 0) {
+    *skip = true;
+    return QTX_OK;
+  }
   if (d.K < 0 || d.nadd < 0 || d.nadd3 < 0 || d.nadd + d.nadd3 > kMaxAddends) {
     set_error("zgemm: invalid sizes or addend count");
     return QTX_ERR_ARG;
@@ -393,21 +401,19 @@ int zgemm(const GemmDesc& d, cudaStream_t s) {
               "and no second outputs");
     return QTX_ERR_ARG;
   }
-  if (!grouped && d.K > 0 && (d.A.null() || d.B.null())) {
+  GemmDesc dd = d;
+  if (!grouped && dd.K > 0 && (dd.A.null() || dd.B.null())) {
     // A zero operand: the product vanishes; only the addends remain.
-    GemmDesc z = d;
-    z.K = 0;
-    z.A = d.C.null() ? d.C3 : d.C;
-    z.B = z.A;
-    return zgemm(z, s);
+    dd.K = 0;
+    dd.A = dd.C.null() ? dd.C3 : dd.C;
+    dd.B = dd.A;
   }
-  if ((d.K > 0 && (!aligned16(d.A) || !aligned16(d.B))) || !aligned16(d.C) || !aligned16(d.C2) ||
-      !aligned16(d.C3)) {
+  if ((dd.K > 0 && (!aligned16(dd.A) || !aligned16(dd.B))) || !aligned16(dd.C) || !aligned16(dd.C2) ||
+      !aligned16(dd.C3)) {
     set_error("zgemm: complex128 operands must be 16-byte aligned");
     return QTX_ERR_ARG;
   }
-  GemmDesc dd = d;
-  for (int t = 0; !grouped && t < d.nadd + d.nadd3; ++t) {
+  for (int t = 0; !grouped && t < dd.nadd + dd.nadd3; ++t) {
     if (dd.add[t].m.null()) {  // drop zero addends
       for (int u = t; u + 1 < dd.nadd + dd.nadd3; ++u) dd.add[u] = dd.add[u + 1];
       if (t < dd.nadd)
@@ -423,21 +429,61 @@ int zgemm(const GemmDesc& d, cudaStream_t s) {
     if (dd.A.null()) dd.A = dd.C.null() ? dd.C3 : dd.C;
     if (dd.B.null()) dd.B = dd.A;
   }
-  if (!grouped && dd.K > 0 && gemm_slices() > 0 && oz_supported(dd.K, gemm_slices())) {
-    size_t bytes = 0;
-    void* scr = oz_bound(&bytes);
-    if (scr != nullptr) return zgemm_oz(dd, gemm_slices(), scr, bytes, s);
-  }
-  KernelArgs args;
-  args.count = 1;
-  args.d[0] = dd;
-  const int key = dd.opA * 2 + dd.opB;
-  switch (key) {
+  *out = dd;
+  return QTX_OK;
+}
+
+bool emulated(const GemmDesc& d, void** scr, size_t* bytes) {
+  if (d.a_ptrs || d.K <= 0 || gemm_slices() <= 0 || !oz_supported(d.K, gemm_slices())) return false;
+  *scr = oz_bound(bytes);
+  return *scr != nullptr;
+}
+
+int dispatch(const KernelArgs& args, cudaStream_t s) {
+  switch (args.d[0].opA * 2 + args.d[0].opB) {
     case 0: return launch<0, 0>(args, s);
     case 1: return launch<0, 1>(args, s);
     case 2: return launch<1, 0>(args, s);
     default: return launch<1, 1>(args, s);
   }
+}
+
+}  // namespace
+
+int zgemm(const GemmDesc& d, cudaStream_t s) { return zgemm_many(&d, 1, s); }
+
+// Consecutive products of the same sizes and operations share a launch: the
+// lesser and greater products of a sweep and the independent products of a
+// step fill the GPU together (a 64-block batch of 32 has 128 tiles a product)
+// and pay one launch and one last wave instead of one each.
+int zgemm_many(const GemmDesc* d, int count, cudaStream_t s) {
+  KernelArgs args;
+  args.count = 0;
+  auto flush = [&]() {
+    const int st = args.count > 0 ? dispatch(args, s) : (int)QTX_OK;
+    args.count = 0;
+    return st;
+  };
+  for (int k = 0; k < count; ++k) {
+    GemmDesc dd;
+    bool skip = false;
+    QTX_TRY(normalize(d[k], &dd, &skip));
+    if (skip) continue;
+    void* scr = nullptr;
+    size_t bytes = 0;
+    if (emulated(dd, &scr, &bytes)) {
+      QTX_TRY(flush());
+      QTX_TRY(zgemm_oz(dd, gemm_slices(), scr, bytes, s));
+      continue;
+    }
+    const GemmDesc& f = args.d[0];
+    if (args.count == kMaxGroup ||
+        (args.count > 0 && (dd.M != f.M || dd.N != f.N || dd.K != f.K || dd.batch != f.batch || dd.opA != f.opA ||
+                            dd.opB != f.opB)))
+      QTX_TRY(flush());
+    args.d[args.count++] = dd;
+  }
+  return flush();
 }
 
 }  // namespace qtx
