@@ -6,12 +6,15 @@
 // Each FP32 operand x is split into x_hi = tf32(x) and x_lo = tf32(x - x_hi);
 // a real product is a_hi b_hi + a_hi b_lo + a_lo b_hi (the lo*lo term is
 // below FP32 rounding). A complex product is the 4M combination of real
-// products, with the subtraction folded into the instruction descriptor's
-// negate bit: 12 tcgen05.mma.kind::tf32 per K step of 8.
+// products. op(B) is staged as the stack [-Bi; Br; Bi], so that with the
+// accumulators [Re | Im] side by side Ar [Br | Bi] and Ai [-Bi | Br] are MMAs
+// of N = 128: six tcgen05.mma.kind::tf32 per K step of 8, which read 48 KB of
+// shared memory where twelve of N = 64 read 72 KB (576 of its cycles against
+// 391 of the tensor pipe).
 //
-// CTA tile 128 x 64 (one UMMA M=128, N=64), K block 32 FP32 (128-byte rows,
-// SWIZZLE_128B K-major), eight warps, one buffer of split planes (96 KB) so
-// that two CTAs share an SM and one's prologue/epilogue overlaps the other's
+// CTA tile 128 x 64 (one UMMA M=128, N=128 real), K block 32 FP32 (128-byte
+// rows, SWIZZLE_128B K-major), eight warps, one buffer of split planes (112 KB)
+// so that two CTAs share an SM and one's prologue/epilogue overlaps the other's
 // MMAs. While the tensor cores run the MMAs of block kb (issued by one
 // thread), all warps load block kb+1 from global memory into registers, wait
 // for the MMAs (tcgen05.commit -> mbarrier), then split and store the planes.
@@ -33,7 +36,8 @@ constexpr int TK = 32;        // fp32 elements per K block (128 B rows)
 constexpr int THREADS = 256;  // eight warps
 constexpr int PLANE_A = TM * TK * 4;  // bytes of one A plane (16 KB)
 constexpr int PLANE_B = TN * TK * 4;  // bytes of one B plane (8 KB)
-constexpr int PLANES_BYTES = 4 * PLANE_A + 4 * PLANE_B;  // re/im x hi/lo for A and B
+// op(A): re/im x hi/lo; op(B): the stack -im, re, im for hi and for lo.
+constexpr int PLANES_BYTES = 4 * PLANE_A + 6 * PLANE_B;
 constexpr int CTAS_PER_SM = 2;                               // one plane buffer each
 constexpr int S_LD = TN + 1;                                 // padded epilogue tile row (float2)
 constexpr int A_TASKS = TM * (TK / 4) / THREADS;             // 4 row-chunks of op(A) per thread
@@ -66,13 +70,12 @@ __device__ __forceinline__ uint64_t make_desc(uint32_t saddr) {
   return d;
 }
 
-// Instruction descriptor: D f32, A/B tf32, K-major both, N = 64, M = 128.
-__host__ __device__ constexpr uint32_t make_idesc(bool neg_a) {
+// Instruction descriptor: D f32, A/B tf32, K-major both, N = 128, M = 128.
+__host__ __device__ constexpr uint32_t make_idesc() {
   return (1u << 4)                  // D format f32
          | (2u << 7)                // A tf32
          | (2u << 10)               // B tf32
-         | ((neg_a ? 1u : 0u) << 13)
-         | ((uint32_t)(TN >> 3) << 17)
+         | ((uint32_t)((2 * TN) >> 3) << 17)
          | ((uint32_t)(TM >> 4) << 24);
 }
 
@@ -259,7 +262,9 @@ __device__ __forceinline__ void split4(const float2 (&v)[4], float4& hr, float4&
   }
 }
 
-// Registers -> the eight split planes (SWIZZLE_128B K-major).
+__device__ __forceinline__ float4 neg4(float4 v) { return make_float4(-v.x, -v.y, -v.z, -v.w); }
+
+// Registers -> the split planes (SWIZZLE_128B K-major).
 template <int OPA, int OPB>
 __device__ __forceinline__ void store_planes(const Regs& R, uint8_t* planes, int tid) {
   uint8_t* pb = planes + 4 * PLANE_A;
@@ -282,52 +287,52 @@ __device__ __forceinline__ void store_planes(const Regs& R, uint8_t* planes, int
     float4 hr, lr, hi, li;
     split4(R.b[i], hr, lr, hi, li);
     const uint32_t off = sw128_offset(row, chunk);
-    *reinterpret_cast<float4*>(pb + off) = hr;
-    *reinterpret_cast<float4*>(pb + PLANE_B + off) = lr;
+    *reinterpret_cast<float4*>(pb + off) = neg4(hi);
+    *reinterpret_cast<float4*>(pb + PLANE_B + off) = hr;
     *reinterpret_cast<float4*>(pb + 2 * PLANE_B + off) = hi;
-    *reinterpret_cast<float4*>(pb + 3 * PLANE_B + off) = li;
+    *reinterpret_cast<float4*>(pb + 3 * PLANE_B + off) = neg4(li);
+    *reinterpret_cast<float4*>(pb + 4 * PLANE_B + off) = lr;
+    *reinterpret_cast<float4*>(pb + 5 * PLANE_B + off) = li;
   }
 }
 
-// The 12 MMAs of one K step (8 fp32) on stage base addresses.
+// The six MMAs of one K step (8 fp32), each over the 128 accumulator columns
+// [Re | Im]: += Ar [Br | Bi] and += Ai [-Bi | Br], small terms first.
 __device__ __forceinline__ void issue_kstep(uint32_t tmem, uint32_t sa, uint32_t sb, int kk,
                                             bool first) {
   const uint32_t koff = (uint32_t)kk * 32;  // bytes along the 128-byte row
   const uint64_t arh = make_desc(sa + 0 * PLANE_A + koff), arl = make_desc(sa + 1 * PLANE_A + koff);
   const uint64_t aih = make_desc(sa + 2 * PLANE_A + koff), ail = make_desc(sa + 3 * PLANE_A + koff);
-  const uint64_t brh = make_desc(sb + 0 * PLANE_B + koff), brl = make_desc(sb + 1 * PLANE_B + koff);
-  const uint64_t bih = make_desc(sb + 2 * PLANE_B + koff), bil = make_desc(sb + 3 * PLANE_B + koff);
-  constexpr uint32_t ID = make_idesc(false), IDN = make_idesc(true);
-  const uint32_t re = tmem, im = tmem + TN;
-  // Re += Ar Br - Ai Bi  (small terms first)
-  mma_tf32(re, arl, brh, ID, first ? 0u : 1u);
-  mma_tf32(re, arh, brl, ID, 1u);
-  mma_tf32(re, arh, brh, ID, 1u);
-  mma_tf32(re, ail, bih, IDN, 1u);
-  mma_tf32(re, aih, bil, IDN, 1u);
-  mma_tf32(re, aih, bih, IDN, 1u);
-  // Im += Ar Bi + Ai Br
-  mma_tf32(im, arl, bih, ID, first ? 0u : 1u);
-  mma_tf32(im, arh, bil, ID, 1u);
-  mma_tf32(im, arh, bih, ID, 1u);
-  mma_tf32(im, ail, brh, ID, 1u);
-  mma_tf32(im, aih, brl, ID, 1u);
-  mma_tf32(im, aih, brh, ID, 1u);
+  const uint64_t bih = make_desc(sb + 0 * PLANE_B + koff), brh = make_desc(sb + 1 * PLANE_B + koff);
+  const uint64_t bil = make_desc(sb + 3 * PLANE_B + koff), brl = make_desc(sb + 4 * PLANE_B + koff);
+  constexpr uint32_t ID = make_idesc();
+  mma_tf32(tmem, arl, brh, ID, first ? 0u : 1u);
+  mma_tf32(tmem, arh, brl, ID, 1u);
+  mma_tf32(tmem, arh, brh, ID, 1u);
+  mma_tf32(tmem, ail, bih, ID, 1u);
+  mma_tf32(tmem, aih, bil, ID, 1u);
+  mma_tf32(tmem, aih, bih, ID, 1u);
 }
 
-__device__ __forceinline__ float2 addend_at(const Args& a, int t, int64_t b, int r, int c) {
-  const auto& ad = a.add[t];
-  const c32* p = at<const c32>(ad.m, b);
-  float2 x = ad.ct ? p[(int64_t)c * ad.m.ld + r] : p[(int64_t)r * ad.m.ld + c];
-  if (ad.ct) x.y = -x.y;
-  return cmulf(ad.coef, x);
+constexpr int PA = 8;  // accumulator columns per epilogue step
+
+// Eight accumulator columns of this lane's row.
+__device__ __forceinline__ void tmem_ld8(uint32_t addr, uint32_t (&v)[PA]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];\n"
+               : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7])
+               : "r"(addr));
 }
+
+constexpr int kMaxGroup = 4;
+struct GroupArgs {
+  int count;
+  Args a[kMaxGroup];
+};
 
 template <int OPA, int OPB, bool VEC>
-__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) cgemm_tc_kernel(const Args a) {
-  extern __shared__ __align__(1024) uint8_t smem_raw[];
+__global__ void __launch_bounds__(THREADS, CTAS_PER_SM) cgemm_tc_kernel(const __grid_constant__ GroupArgs ga) {
   // 1024-byte alignment for the SWIZZLE_128B atoms.
-  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) uint8_t smem[];
   uint8_t* planes = smem;
   float2* tile = reinterpret_cast<float2*>(smem);  // epilogue tile [TM][S_LD], reuses the planes
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + PLANES_BYTES);
@@ -338,7 +343,8 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) cgemm_tc_kernel(const Ar
   const int lane = tid & 31;
   const int m0 = blockIdx.y * TM;
   const int n0 = blockIdx.x * TN;
-  const int KB = (a.K + TK - 1) / TK;
+  const int64_t batch = ga.a[0].batch;
+  const int KB = (ga.a[0].K + TK - 1) / TK;
 
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;\n" ::"r"(
@@ -357,12 +363,11 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) cgemm_tc_kernel(const Ar
   uint32_t phase = 0;
   bool ok = true;
   Regs R;
-  // Addends split by orientation: conjugate-transposed ones are read with
-  // lanes along rows (phase A), the others with lanes along columns (phase B).
-  int n_ct = 0;
-  for (int t = 0; t < a.nadd; ++t) n_ct += a.add[t].ct;
 
-  for (int64_t b = blockIdx.z; b < a.batch && ok; b += gridDim.z) {
+  for (int64_t z = blockIdx.z; z < batch * ga.count && ok; z += gridDim.z) {
+    const int set = (int)(z / batch);
+    const int64_t b = z - set * batch;
+    const Args& a = ga.a[set];
     const c32* Ag = at<const c32>(a.A, b);
     const c32* Bg = at<const c32>(a.B, b);
     if (KB > 0) {
@@ -408,100 +413,140 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) cgemm_tc_kernel(const Ar
       const uint32_t lane_base = tmem + ((uint32_t)(wl * 32) << 16);
       const int cbeg = (warp >> 2) * (TN / 2);
 #pragma unroll 1
-      for (int c0 = cbeg; c0 < cbeg + TN / 2; c0 += 16) {
-        uint32_t vr[16], vi[16];
+      for (int c0 = cbeg; c0 < cbeg + TN / 2; c0 += PA) {
+        uint32_t vr[PA], vi[PA];
         if (KB > 0) {
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-              : "=r"(vr[0]), "=r"(vr[1]), "=r"(vr[2]), "=r"(vr[3]), "=r"(vr[4]), "=r"(vr[5]),
-                "=r"(vr[6]), "=r"(vr[7]), "=r"(vr[8]), "=r"(vr[9]), "=r"(vr[10]), "=r"(vr[11]),
-                "=r"(vr[12]), "=r"(vr[13]), "=r"(vr[14]), "=r"(vr[15])
-              : "r"(lane_base + (uint32_t)c0));
-          asm volatile(
-              "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n"
-              : "=r"(vi[0]), "=r"(vi[1]), "=r"(vi[2]), "=r"(vi[3]), "=r"(vi[4]), "=r"(vi[5]),
-                "=r"(vi[6]), "=r"(vi[7]), "=r"(vi[8]), "=r"(vi[9]), "=r"(vi[10]), "=r"(vi[11]),
-                "=r"(vi[12]), "=r"(vi[13]), "=r"(vi[14]), "=r"(vi[15])
-              : "r"(lane_base + (uint32_t)(TN + c0)));
+          tmem_ld8(lane_base + (uint32_t)c0, vr);
+          tmem_ld8(lane_base + (uint32_t)(TN + c0), vi);
           asm volatile("tcgen05.wait::ld.sync.aligned;\n" ::);
         } else {
 #pragma unroll
-          for (int j = 0; j < 16; ++j) vr[j] = vi[j] = 0u;
+          for (int j = 0; j < PA; ++j) vr[j] = vi[j] = 0u;
+        }
+        float2 v[PA];
+#pragma unroll
+        for (int j = 0; j < PA; ++j)
+          v[j] = cmulf(a.alpha, make_float2(__uint_as_float(vr[j]), __uint_as_float(vi[j])));
+        for (int t = 0; t < a.nadd; ++t) {
+          const auto& ad = a.add[t];
+          if (!ad.ct) continue;
+          const c32* p = at<const c32>(ad.m, b) + (int64_t)(n0 + c0) * ad.m.ld + r;
+          float2 x[PA];  // all loads first
+#pragma unroll
+          for (int j = 0; j < PA; ++j)
+            x[j] = (r < a.M && n0 + c0 + j < a.N) ? p[(int64_t)j * ad.m.ld] : make_float2(0.f, 0.f);
+#pragma unroll
+          for (int j = 0; j < PA; ++j) {
+            const float2 y = cmulf(ad.coef, make_float2(x[j].x, -x[j].y));
+            v[j].x += y.x;
+            v[j].y += y.y;
+          }
         }
 #pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const int c = n0 + c0 + j;
-          float2 v = cmulf(a.alpha, make_float2(__uint_as_float(vr[j]), __uint_as_float(vi[j])));
-          if (n_ct > 0 && r < a.M && c < a.N) {
-            for (int t = 0; t < a.nadd; ++t) {
-              if (!a.add[t].ct) continue;
-              const float2 y = addend_at(a, t, b, r, c);
-              v.x += y.x;
-              v.y += y.y;
-            }
-          }
-          tile[rl * S_LD + c0 + j] = v;
-        }
+        for (int j = 0; j < PA; ++j) tile[rl * S_LD + c0 + j] = v[j];
       }
     }
     asm volatile("tcgen05.fence::before_thread_sync;\n" ::);
     __syncthreads();
 
-    // Phase B (lane = tile column): remaining addends, C3 and C.
+    // Phase B (a warp takes four rows at a time, lane = tile column and
+    // column + 32): the addends read row-wise, C3 and C. All loads of an
+    // addend are issued before their use: one element at a time (as before)
+    // exposed a memory latency per element and addend, 180 us for an NT product
+    // of 64 x 256^3 with addends against 104 us without.
+    constexpr int PB = 4;
 #pragma unroll 1
-    for (int e = tid; e < TM * TN; e += THREADS) {
-      const int rl = e / TN, cl = e % TN;
-      const int r = m0 + rl, c = n0 + cl;
-      if (r >= a.M || c >= a.N) continue;
-      float2 v = tile[rl * S_LD + cl];
-      for (int t = 0; t < a.nadd; ++t) {
-        if (a.add[t].ct) continue;
-        const float2 y = addend_at(a, t, b, r, c);
-        v.x += y.x;
-        v.y += y.y;
-      }
+    for (int rb = warp * PB; rb < TM; rb += (THREADS / 32) * PB) {
+      if (m0 + rb >= a.M) break;
+      float2 v[PB][2];
+      auto inside = [&](int k, int h) { return m0 + rb + k < a.M && n0 + lane + 32 * h < a.N; };
+      auto add_rows = [&](int t, float2(&w)[PB][2]) {
+        const auto& ad = a.add[t];
+        const int64_t rs = ad.ct ? 1 : ad.m.ld, cs = ad.ct ? ad.m.ld : 1;
+        const c32* p = at<const c32>(ad.m, b) + (m0 + rb) * rs + (n0 + lane) * cs;
+        float2 x[PB][2];
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            x[k][h] = inside(k, h) ? p[k * rs + 32 * h * cs] : make_float2(0.f, 0.f);
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const float2 y = cmulf(ad.coef, make_float2(x[k][h].x, ad.ct ? -x[k][h].y : x[k][h].y));
+            w[k][h].x += y.x;
+            w[k][h].y += y.y;
+          }
+      };
+#pragma unroll
+      for (int k = 0; k < PB; ++k)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) v[k][h] = tile[(rb + k) * S_LD + lane + 32 * h];
+      for (int t = 0; t < a.nadd; ++t)
+        if (!a.add[t].ct) add_rows(t, v);
       if (!a.C3.null()) {
-        float2 v3 = cmulf(a.scale3, v);
-        for (int t = a.nadd; t < a.nadd + a.nadd3; ++t) {
-          const float2 y = addend_at(a, t, b, r, c);
-          v3.x += y.x;
-          v3.y += y.y;
-        }
-        at<c32>(a.C3, b)[(int64_t)r * a.C3.ld + c] = v3;
+        float2 w[PB][2];
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) w[k][h] = cmulf(a.scale3, v[k][h]);
+        for (int t = a.nadd; t < a.nadd + a.nadd3; ++t) add_rows(t, w);
+        c32* out = at<c32>(a.C3, b) + (int64_t)(m0 + rb) * a.C3.ld + n0 + lane;
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            if (inside(k, h)) out[(int64_t)k * a.C3.ld + 32 * h] = w[k][h];
       }
-      if (!a.C.null()) at<c32>(a.C, b)[(int64_t)r * a.C.ld + c] = v;
-      if (!a.C2.null()) tile[rl * S_LD + cl] = v;
+      if (!a.C.null()) {
+        c32* out = at<c32>(a.C, b) + (int64_t)(m0 + rb) * a.C.ld + n0 + lane;
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+            if (inside(k, h)) out[(int64_t)k * a.C.ld + 32 * h] = v[k][h];
+      }
+      if (!a.C2.null()) {
+#pragma unroll
+        for (int k = 0; k < PB; ++k)
+#pragma unroll
+          for (int h = 0; h < 2; ++h) tile[(rb + k) * S_LD + lane + 32 * h] = v[k][h];
+      }
     }
 
     // Phase C (lane = tile row): the conjugate-transposed store C2.
     if (!a.C2.null()) {
       __syncthreads();
-#pragma unroll 1
+      c32* out = at<c32>(a.C2, b);
+#pragma unroll 8
       for (int e = tid; e < TM * TN; e += THREADS) {
         const int rl = e % TM, cl = e / TM;
         const int r = m0 + rl, c = n0 + cl;
         if (r >= a.M || c >= a.N) continue;
         const float2 v = tile[rl * S_LD + cl];
-        at<c32>(a.C2, b)[(int64_t)c * a.C2.ld + r] = cmulf(a.coef2, make_float2(v.x, -v.y));
+        out[(int64_t)c * a.C2.ld + r] = cmulf(a.coef2, make_float2(v.x, -v.y));
       }
     }
     __syncthreads();
   }
-  if (!ok && tid == 0 && a.err != nullptr) atomicExch(a.err, 1);
+  if (!ok && tid == 0 && ga.a[0].err != nullptr) atomicExch(ga.a[0].err, 1);
   __syncthreads();
   if (warp == 0)
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;\n" ::"r"(tmem), "r"(TMEM_COLS));
 }
 
 template <int OPA, int OPB, bool VEC>
-int launch_v(const Args& a, cudaStream_t s) {
+int launch_v(const GroupArgs& ga, cudaStream_t s) {
   static_assert(TM * S_LD * (int)sizeof(float2) <= PLANES_BYTES, "epilogue tile must fit the planes");
-  const size_t smem = (size_t)PLANES_BYTES + 64 + 1024;
+  const Args& a = ga.a[0];
+  const size_t smem = (size_t)PLANES_BYTES + 64;
   QTX_CHECK_CUDA(cudaFuncSetAttribute(cgemm_tc_kernel<OPA, OPB, VEC>,
                                       cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  dim3 grid((a.N + TN - 1) / TN, (a.M + TM - 1) / TM, (unsigned)(a.batch < 65535 ? a.batch : 65535));
-  ProfScope prof(QTX_KERNEL_CGEMM, 8.0 * a.M * a.N * (double)a.K * (double)a.batch, s);
-  cgemm_tc_kernel<OPA, OPB, VEC><<<grid, THREADS, smem, s>>>(a);
+  const int64_t z = a.batch * ga.count;
+  dim3 grid((a.N + TN - 1) / TN, (a.M + TM - 1) / TM, (unsigned)(z < 65535 ? z : 65535));
+  ProfScope prof(QTX_KERNEL_CGEMM, 8.0 * a.M * a.N * (double)a.K * (double)z, s);
+  cgemm_tc_kernel<OPA, OPB, VEC><<<grid, THREADS, smem, s>>>(ga);
   QTX_CHECK_LAUNCH();
   return QTX_OK;
 }
@@ -511,58 +556,82 @@ bool vec_ok(const MatRef& m) {
 }
 
 template <int OPA, int OPB>
-int launch(const Args& a, cudaStream_t s) {
-  // The 16-byte path reads the K-contiguous operands; both must allow it.
-  const bool va = OPA != 0 || vec_ok(a.A);
-  const bool vb = OPB != 1 || vec_ok(a.B);
-  if (va && vb) return launch_v<OPA, OPB, true>(a, s);
-  return launch_v<OPA, OPB, false>(a, s);
+int launch(const GroupArgs& ga, cudaStream_t s) {
+  // The 16-byte path reads the K-contiguous operands; all must allow it.
+  bool vec = true;
+  for (int k = 0; k < ga.count; ++k)
+    vec = vec && (OPA != 0 || vec_ok(ga.a[k].A)) && (OPB != 1 || vec_ok(ga.a[k].B));
+  if (vec) return launch_v<OPA, OPB, true>(ga, s);
+  return launch_v<OPA, OPB, false>(ga, s);
+}
+
+int dispatch(const GroupArgs& ga, int op, cudaStream_t s) {
+  switch (op) {
+    case 0: return launch<0, 0>(ga, s);
+    case 1: return launch<0, 1>(ga, s);
+    case 2: return launch<1, 0>(ga, s);
+    default: return launch<1, 1>(ga, s);
+  }
 }
 
 }  // namespace
 
-int cgemm_tc(const CGemmDesc& d, cudaStream_t s) {
-  if (d.M <= 0 || d.N <= 0 || d.batch <= 0) return QTX_OK;
-  if (d.nadd < 0 || d.nadd3 < 0 || d.nadd + d.nadd3 > kMaxAddends ||
-      (d.K > 0 && (d.A.null() || d.B.null())) || (d.C.null() && d.C3.null())) {
-    set_error("cgemm_tc: invalid arguments (null operand or output, or too many addends)");
-    return QTX_ERR_ARG;
+int cgemm_tc(const CGemmDesc& d, cudaStream_t s) { return cgemm_tc_many(&d, 1, s); }
+
+// As zgemm_many: consecutive products of one shape share a launch.
+int cgemm_tc_many(const CGemmDesc* list, int count, cudaStream_t s) {
+  GroupArgs ga;
+  ga.count = 0;
+  int op = 0;
+  auto flush = [&]() {
+    const int st = ga.count > 0 ? dispatch(ga, op, s) : (int)QTX_OK;
+    ga.count = 0;
+    return st;
+  };
+  for (int i = 0; i < count; ++i) {
+    const CGemmDesc& d = list[i];
+    if (d.M <= 0 || d.N <= 0 || d.batch <= 0) continue;
+    if (d.nadd < 0 || d.nadd3 < 0 || d.nadd + d.nadd3 > kMaxAddends ||
+        (d.K > 0 && (d.A.null() || d.B.null())) || (d.C.null() && d.C3.null())) {
+      set_error("cgemm_tc: invalid arguments (null operand or output, or too many addends)");
+      return QTX_ERR_ARG;
+    }
+    const Args& f = ga.a[0];
+    if (ga.count == kMaxGroup ||
+        (ga.count > 0 && (d.M != f.M || d.N != f.N || d.K != f.K || d.batch != f.batch || d.err != f.err ||
+                          d.opA * 2 + d.opB != op)))
+      QTX_TRY(flush());
+    op = d.opA * 2 + d.opB;
+    Args a{};
+    a.M = d.M;
+    a.N = d.N;
+    a.K = d.K;
+    a.batch = d.batch;
+    a.A = d.A;
+    a.B = d.B;
+    a.opA = d.opA;
+    a.opB = d.opB;
+    a.alpha = d.alpha;
+    for (int t = 0; t < d.nadd + d.nadd3; ++t) {
+      if (d.add[t].m.null()) continue;
+      const int k = a.nadd + a.nadd3;
+      a.add[k].m = d.add[t].m;
+      a.add[k].coef = d.add[t].coef;
+      a.add[k].ct = d.add[t].conj_trans;
+      if (t < d.nadd)
+        ++a.nadd;
+      else
+        ++a.nadd3;
+    }
+    a.C = d.C;
+    a.C2 = d.C2;
+    a.C3 = d.C3;
+    a.coef2 = d.coef2;
+    a.scale3 = d.scale3;
+    a.err = d.err;
+    ga.a[ga.count++] = a;
   }
-  Args a{};
-  a.M = d.M;
-  a.N = d.N;
-  a.K = d.K;
-  a.batch = d.batch;
-  a.A = d.A;
-  a.B = d.B;
-  a.opA = d.opA;
-  a.opB = d.opB;
-  a.alpha = d.alpha;
-  a.nadd = 0;
-  a.nadd3 = 0;
-  for (int t = 0; t < d.nadd + d.nadd3; ++t) {
-    if (d.add[t].m.null()) continue;
-    const int k = a.nadd + a.nadd3;
-    a.add[k].m = d.add[t].m;
-    a.add[k].coef = d.add[t].coef;
-    a.add[k].ct = d.add[t].conj_trans;
-    if (t < d.nadd)
-      ++a.nadd;
-    else
-      ++a.nadd3;
-  }
-  a.C = d.C;
-  a.C2 = d.C2;
-  a.C3 = d.C3;
-  a.coef2 = d.coef2;
-  a.scale3 = d.scale3;
-  a.err = d.err;
-  switch (d.opA * 2 + d.opB) {
-    case 0: return launch<0, 0>(a, s);
-    case 1: return launch<0, 1>(a, s);
-    case 2: return launch<1, 0>(a, s);
-    default: return launch<1, 1>(a, s);
-  }
+  return flush();
 }
 
 }  // namespace qtx

@@ -155,6 +155,7 @@ struct CGemmDesc {
   int* err = nullptr;  // set to 1 if an mbarrier wait timed out
 };
 int cgemm_tc(const CGemmDesc& d, cudaStream_t s);
+int cgemm_tc_many(const CGemmDesc* d, int count, cudaStream_t s);  // see zgemm_many
 
 // Batched in-place Gauss-Jordan inversion with partial pivoting (zinv.cu).
 // X <- A^{-1} for each of `batch` n x n matrices; X may alias A. `info[b]`

@@ -251,8 +251,14 @@ struct MixedGemm {
 };
 
 int run_all(std::vector<MixedGemm> list, cudaStream_t s) {
-  for (MixedGemm& g : list) QTX_TRY(g.run(s));
-  return QTX_OK;
+  std::vector<CGemmDesc> d;
+  for (MixedGemm& g : list) {
+    if (g.d.K > 0 && (g.d.A.null() || g.d.B.null()))
+      QTX_TRY(g.run(s));  // a zero operand: a combine
+    else
+      d.push_back(g.d);
+  }
+  return cgemm_tc_many(d.data(), (int)d.size(), s);
 }
 
 struct Mixed {
