@@ -115,12 +115,11 @@ __device__ __forceinline__ int gj_best_lane(unsigned long long key, int pos) {
 // of the CTA take part and the others return at once (named barrier 1).
 // load(r, c) / store(r, c, v): panel element access (r < n, c < nbp), the same
 // memory or not (a barrier separates loads and stores); moved(r, pos), once per
-// row after that barrier: row r ends at position pos; pivot(k, p), by one
-// thread: position p was chosen for column k. sing: shared int, set to k + 1 at
-// the first zero pivot if still 0.
-template <int NB, class Load, class Store, class Moved, class Pivot>
+// row after that barrier: row r ends at position pos. sing: shared int, set to
+// k + 1 at the first zero pivot if still 0.
+template <int NB, class Load, class Store, class Moved>
 __device__ __forceinline__ void gj_factor_panel(int n, int k0, int nbp, Load load, Store store, Moved moved,
-                                                Pivot pivot, int* sing) {
+                                                int* sing) {
   __shared__ GjPanelSmem<NB> sm;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int W = (n + 31) >> 5;
@@ -172,7 +171,6 @@ __device__ __forceinline__ void gj_factor_panel(int n, int k0, int nbp, Load loa
     z64 m = gj_mul(v[0], d);
     if (piv) {
       // the scaled pivot row q / x_pk as 0 - (-1 / x_pk) q
-      pivot(k, p);
       if (sm.key[wl] <= 1ull && *sing == 0) *sing = k + 1;
 #pragma unroll
       for (int c = 1; c < NB; ++c) v[c] = make_double2(0.0, 0.0);

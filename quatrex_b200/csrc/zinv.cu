@@ -790,7 +790,7 @@ __global__ void __launch_bounds__(TH, 512 / TH) zinv3_kernel(int n, int64_t batc
             srcrow[pos] = r;
             orig[(cur ^ 1) * np + pos] = orig[cur * np + r];
           },
-          [](int, int) {}, &s_sing);
+          &s_sing);
       cur ^= 1;
       __syncthreads();
       // 2. Pivot rows of this CTA's other columns; the transform into X[:, K].

@@ -18,11 +18,11 @@
 //           swizzle, no multicast) into four [rows][8 complex] chunks;
 //   panel:  the CTA owning the 16 columns of panel K factors them in place
 //           (gj_panel.cuh), then arrives on the cluster barrier;
-//   update: every CTA reads the panel transform T = X[:, K] and the pivot
-//           rows from the owner's shared memory (DSMEM), applies the row
-//           interchanges to its own columns and updates them,
-//             X[r, J] = (r in K ? 0 : X[r, J]) + T[r, :] X[K, J],
-//           with FP64 tensor-core MMAs (mma.sync m16n8k4, 4M complex split);
+//   update: every CTA receives the panel transform T = X[:, K] and the row
+//           moves from the owner (bulk copies) and updates its own columns,
+//             X[r, J] = (r in K ? 0 : X[src(r), J]) + T[r, :] Y[:, J],
+//           Y = X[src(K), J], with FP64 tensor-core MMAs (mma.sync m16n8k4, 4M
+//           complex split); src carries the row interchanges;
 //   store:  columns are gathered back through DSMEM in the inverse column
 //           order of the pivoting and written with coalesced stores.
 //
@@ -84,14 +84,15 @@ __device__ __forceinline__ int xoff(int npad, int r, int j) {
 struct ClusterSmem {
   // byte offsets inside the dynamic shared memory (base aligned to 1024)
   int npad;
-  size_t x, t, y, piv, colsrc, bar, total;
+  size_t x, t, y, src, orig, colsrc, bar, total;
   __host__ __device__ explicit ClusterSmem(int n) {
     npad = (n + 15) & ~15;
     x = 0;                                                  // 4 chunks [npad][8]
     t = x + (size_t)4 * npad * 8 * sizeof(z64);             // 2 chunks [npad][8]
     y = t + (size_t)2 * npad * 8 * sizeof(z64);             // [CNB][YS]
-    piv = y + (size_t)CNB * YS * sizeof(z64);               // npad ints
-    colsrc = piv + (size_t)npad * sizeof(int);              // npad ints
+    src = y + (size_t)CNB * YS * sizeof(z64);               // 2 x npad ints
+    orig = src + (size_t)2 * npad * sizeof(int);            // 2 x npad ints
+    colsrc = orig + (size_t)2 * npad * sizeof(int);         // npad ints
     bar = (colsrc + (size_t)npad * sizeof(int) + 15) & ~(size_t)15;  // 2 mbarriers
     total = bar + 16 + 1024;  // + alignment slack of the base
   }
@@ -135,7 +136,10 @@ __global__ void __launch_bounds__(CT, 1)
   z64* Xs = reinterpret_cast<z64*>(base + L.x);
   z64* Ts = reinterpret_cast<z64*>(base + L.t);
   z64* Ys = reinterpret_cast<z64*>(base + L.y);
-  int* pivrow = reinterpret_cast<int*>(base + L.piv);
+  // row of X that each position receives, by panel parity: the owner may factor
+  // the next panel while this one's copies to the others are in flight
+  int* const srcbuf = reinterpret_cast<int*>(base + L.src);
+  int* orig = reinterpret_cast<int*>(base + L.orig);   // original row of each position (2 buffers)
   int* colsrc = reinterpret_cast<int*>(base + L.colsrc);
   uint64_t* lbar = reinterpret_cast<uint64_t*>(base + L.bar);  // the load of A
   uint64_t* tbar = lbar + 1;                                    // the panel transforms
@@ -147,6 +151,7 @@ __global__ void __launch_bounds__(CT, 1)
   const size_t chunk = (size_t)npad * 8;  // complex elements per 8-column chunk
 
   // ---- load this CTA's 32 columns --------------------------------------
+  for (int r = tid; r < npad; r += CT) srcbuf[r] = srcbuf[npad + r] = orig[r] = r;
   if (tid == 0) {
     s_sing = 0;
     s_first = 0x7fffffff;
@@ -184,17 +189,19 @@ __global__ void __launch_bounds__(CT, 1)
 
   // ---- panels -----------------------------------------------------------
   uint32_t tphase = 0;
+  int cur = 0;
   for (int k0 = 0; k0 < n; k0 += CNB) {
     const int owner = k0 / CW, kl = k0 - owner * CW;
     const int nbp = min(CNB, n - k0);
     const bool own = rank == owner;
-    const uint32_t tbytes = (uint32_t)(2 * chunk * sizeof(z64)) + CNB * sizeof(int);
+    int* const srcrow = srcbuf + ((k0 / CNB) & 1) * npad;
+    const uint32_t tbytes = (uint32_t)(2 * chunk * sizeof(z64)) + (uint32_t)npad * sizeof(int);
 
     if (own) {
       gj_factor_panel<CNB>(
           n, k0, nbp, [=](int r, int c) { return Xs[xoff(npad, r, kl + c)]; },
-          [=](int r, int c, z64 v) { Xs[xoff(npad, r, kl + c)] = v; }, [](int, int) {},
-          [=](int k, int p) { pivrow[k] = p; }, &s_sing);
+          [=](int r, int c, z64 v) { Xs[xoff(npad, r, kl + c)] = v; },
+          [=](int r, int pos) { srcrow[pos] = r; }, &s_sing);
       // the panel's stores must be visible to the bulk copies below
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
     } else if (tid == 0) {
@@ -206,10 +213,10 @@ __global__ void __launch_bounds__(CT, 1)
     cluster_arrive();
     cluster_wait();
     if (own && tid == 0) {
-      // The transform (columns kl..kl+15: two whole chunks) and its pivots
+      // The transform (columns kl..kl+15: two whole chunks) and the row moves
       // to every other CTA of the cluster (bulk copies, no multicast).
       const uint32_t src_t = saddr(Xs + (size_t)(kl >> 3) * chunk);
-      const uint32_t src_p = saddr(pivrow + k0);
+      const uint32_t src_p = saddr(srcrow);
       for (int r = 0; r < C; ++r) {
         if (r == rank) continue;
         const uint32_t mb = cluster_addr(saddr(tbar), r);
@@ -220,8 +227,8 @@ __global__ void __launch_bounds__(CT, 1)
             : "memory");
         asm volatile(
             "cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];\n" ::"r"(
-                cluster_addr(saddr(pivrow + k0), r)),
-            "r"(src_p), "r"((uint32_t)(CNB * sizeof(int))), "r"(mb)
+                cluster_addr(saddr(srcrow), r)),
+            "r"(src_p), "r"((uint32_t)(npad * sizeof(int))), "r"(mb)
             : "memory");
       }
     }
@@ -232,89 +239,68 @@ __global__ void __launch_bounds__(CT, 1)
     }
     const z64* T = own ? Xs + (size_t)(kl >> 3) * chunk : Ts;
 
-    // Row interchanges of this CTA's other columns (lane = column), then the
-    // pivot rows Y.
-    if (warp == 0) {
-      const int j = lane;
-      const bool panel = own && j >= kl && j < kl + CNB;
-      if (!panel) {
-        for (int kk = 0; kk < nbp; ++kk) {
-          const int k = k0 + kk, p = pivrow[k];
-          if (p != k) {
-            const z64 a = Xs[xoff(npad, k, j)], c = Xs[xoff(npad, p, j)];
-            Xs[xoff(npad, k, j)] = c;
-            Xs[xoff(npad, p, j)] = a;
-          }
-        }
-      }
-#pragma unroll
-      for (int kk = 0; kk < CNB; ++kk)
-        Ys[kk * YS + j] = (kk < nbp && !panel) ? Xs[xoff(npad, k0 + kk, j)] : make_double2(0.0, 0.0);
+    // Pivot rows of this CTA's other columns, one element per thread.
+    {
+      const int kk = tid / CW, j = tid % CW;
+      const bool use = kk < nbp && !(own && j >= kl && j < kl + CNB);
+      Ys[kk * YS + j] = use ? Xs[xoff(npad, srcrow[k0 + kk], j)] : make_double2(0.0, 0.0);
     }
+    for (int r = tid; r < n; r += CT) orig[(cur ^ 1) * npad + r] = orig[cur * npad + srcrow[r]];
+    cur ^= 1;
     __syncthreads();
 
-    // Update: warp w takes rows [16 w, 16 w + 16) of a pair of 8-column
-    // tiles at a time (four independent accumulator chains); the owner skips
-    // the pair that holds the panel (kl is 0 or 16: exactly one pair).
-    const int mtiles = (n + 15) >> 4;
-    for (int mt = warp; mt < mtiles; mt += CWARPS) {
-      const int r0 = mt * 16;
-      const int ra = r0 + g;
-#pragma unroll 1
-      for (int jp = 0; jp < 2; ++jp) {
-        if (own && jp * 16 == kl) continue;
-        double cre[2][4], cim[2][4];
+    // Update in tiles of 16 rows x 8 columns dealt to the warps, the owner
+    // without the panel's two: first the slices other than the pivots', from
+    // the rows that LAPACK's interchanges would have brought there, then (those
+    // read rows of K) the pivots'. One warp applying the interchanges ahead of
+    // an update of whole 16-row slices took 18 of 37 kcycles per panel at
+    // n = 128.
+    const int mtiles = npad >> 4, kt = k0 / CNB, nt = own ? 2 : 4;
+    for (int phase = 0; phase < 2; ++phase) {
+      const int units = phase == 0 ? (mtiles - 1) * nt : nt;
+      for (int u = warp; u < units; u += CWARPS) {
+        int mt = u / nt, jt = u % nt;
+        if (phase == 1)
+          mt = kt;
+        else if (mt >= kt)
+          ++mt;
+        if (own && jt * 8 >= kl) jt += 2;
+        const int ra = mt * 16 + g;
+        const int q0 = srcrow[ra], q1 = srcrow[ra + 8];
+        double cre[4], cim[4];
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int r = ra + ((q >> 1) << 3);
-            const int j = jp * 16 + t * 8 + 2 * tq + (q & 1);
-            z64 v = make_double2(0.0, 0.0);
-            if (r < n && !(r >= k0 && r < k0 + nbp)) v = Xs[xoff(npad, r, j)];
-            cre[t][q] = v.x;
-            cim[t][q] = v.y;
-          }
+        for (int q = 0; q < 4; ++q) {
+          z64 v = make_double2(0.0, 0.0);
+          if (phase == 0) v = Xs[xoff(npad, (q >> 1) ? q1 : q0, jt * 8 + 2 * tq + (q & 1))];
+          cre[q] = v.x;
+          cim[q] = v.y;
+        }
 #pragma unroll
         for (int k4 = 0; k4 < CNB; k4 += 4) {
           const int ka = k4 + tq;
           const z64 v0 = T[(ka >> 3) * chunk + ra * 8 + ((ka & 7) ^ (ra & 7))];
           const z64 v1 = T[(ka >> 3) * chunk + (ra + 8) * 8 + ((ka & 7) ^ ((ra + 8) & 7))];
-#pragma unroll
-          for (int t = 0; t < 2; ++t) {
-            const z64 bv = Ys[ka * YS + jp * 16 + t * 8 + g];
-            mma_f64(cre[t], v0.x, v1.x, bv.x);
-            mma_f64(cim[t], v0.x, v1.x, bv.y);
-            mma_f64(cre[t], -v0.y, -v1.y, bv.y);
-            mma_f64(cim[t], v0.y, v1.y, bv.x);
-          }
+          const z64 bv = Ys[ka * YS + jt * 8 + g];
+          mma_f64(cre, v0.x, v1.x, bv.x);
+          mma_f64(cim, v0.x, v1.x, bv.y);
+          mma_f64(cre, -v0.y, -v1.y, bv.y);
+          mma_f64(cim, v0.y, v1.y, bv.x);
         }
 #pragma unroll
-        for (int t = 0; t < 2; ++t)
-#pragma unroll
-          for (int q = 0; q < 4; ++q) {
-            const int r = ra + ((q >> 1) << 3);
-            const int j = jp * 16 + t * 8 + 2 * tq + (q & 1);
-            if (r < n) Xs[xoff(npad, r, j)] = make_double2(cre[t][q], cim[t][q]);
-          }
+        for (int q = 0; q < 4; ++q) {
+          const int r = ra + ((q >> 1) << 3);
+          if (r < n) Xs[xoff(npad, r, jt * 8 + 2 * tq + (q & 1))] = make_double2(cre[q], cim[q]);
+        }
       }
+      __syncthreads();
     }
-    __syncthreads();
   }
 
   // ---- column permutation and store --------------------------------------
-  // Output column q is column colsrc[q] of the Gauss-Jordan result (the
-  // panel interchanges undone from the last pivot back).
+  // Position s holds original row orig[s]: column s of the Gauss-Jordan result
+  // is column orig[s] of the inverse.
+  for (int s = tid; s < n; s += CT) colsrc[orig[cur * npad + s]] = s;
   if (tid == 0) {
-    for (int c = 0; c < n; ++c) colsrc[c] = c;
-    for (int k = n - 1; k >= 0; --k) {
-      const int p = pivrow[k];
-      if (p != k) {
-        const int t = colsrc[k];
-        colsrc[k] = colsrc[p];
-        colsrc[p] = t;
-      }
-    }
     if (s_sing != 0) atomicMin(cluster.map_shared_rank(&s_first, 0), s_sing);
   }
   __syncthreads();
