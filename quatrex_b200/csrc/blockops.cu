@@ -101,6 +101,7 @@ __global__ void __launch_bounds__(TILE* ROWS)
     antiherm_kernel(int n, int64_t batch, int count, const AntihermArgs args, double* density, int64_t ds,
                     int64_t doff) {
   __shared__ z64 tile[TILE][TILE + 1];
+  chain_begin();
   const int c0 = blockIdx.x * TILE, r0 = blockIdx.y * TILE;
   const int tx = threadIdx.x, ty = threadIdx.y;
   for (int64_t z = blockIdx.z; z < batch * count; z += gridDim.z) {
@@ -189,6 +190,7 @@ __global__ void __launch_bounds__(RT) trace_kernel(int n, int64_t batch, const T
   __shared__ double red[RT / 32];
   __shared__ double part[kChunks][4];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  chain_begin();
   cg::cluster_group cluster = cg::this_cluster();
   const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int64_t b = blockIdx.x / S;  // uniform within a cluster
@@ -248,6 +250,7 @@ __global__ void __launch_bounds__(RT) reduce_kernel(int m, int n, int64_t batch,
                                                     const int* active) {
   __shared__ double red[RT / 32];
   __shared__ double part[kChunks][V];
+  chain_begin();
   cg::cluster_group cluster = cg::this_cluster();
   const int S = (int)cluster.num_blocks(), rank = (int)cluster.block_rank();
   const int64_t b = blockIdx.x / S;
@@ -326,32 +329,21 @@ __global__ void convert_kernel(int m, int n, int64_t batch, MatRef in, MatRef ou
 
 unsigned grid_z(int64_t batch) { return (unsigned)(batch < 65535 ? batch : 65535); }
 
-// Cluster launch of one reduction: CTAs per entry, a power of two up to
-// kChunks while all CTAs of the batch are resident at once (8 per SM).
-cudaLaunchConfig_t cluster_config(int64_t batch, cudaLaunchAttribute* attr, cudaStream_t s) {
+// CTAs (a cluster) per entry of a reduction: a power of two up to kChunks while
+// all CTAs of the batch are resident at once (8 per SM).
+int reduce_split(int64_t batch) {
   int S = 1;
   while (S < kChunks && batch * S * 2 <= 8 * (int64_t)num_sms()) S *= 2;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(batch * S), 1, 1);
-  cfg.blockDim = dim3(RT, 1, 1);
-  cfg.stream = s;
-  attr->id = cudaLaunchAttributeClusterDimension;
-  attr->val.clusterDim.x = (unsigned)S;
-  attr->val.clusterDim.y = 1;
-  attr->val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  return cfg;
+  return S;
 }
 
 template <typename T, int V, class F, class Done>
 int reduce_t(int m, int n, int64_t batch, MatRef X, MatRef Y, F f, Done done, const int* active, cudaStream_t s) {
   if (m <= 0 || n <= 0 || batch <= 0) return QTX_OK;
   ProfScope prof(QTX_KERNEL_REDUCE, 2.0 * sizeof(T) * m * n * (double)batch, s);
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = cluster_config(batch, &attr, s);
-  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, reduce_kernel<T, V, F, Done>, m, n, batch, X, Y, f, done, active));
-  return QTX_OK;
+  const int S = reduce_split(batch);
+  return launch_chained(reduce_kernel<T, V, F, Done>, dim3((unsigned)(batch * S)), dim3(RT), 0, s, S, m, n, batch, X, Y,
+                        f, done, active);
 }
 
 template <typename T>
@@ -391,9 +383,8 @@ int antiherm_t(int n, int64_t batch, int count, const MatRef* X, const MatRef* o
   }
   dim3 grid((n + TILE - 1) / TILE, (n + TILE - 1) / TILE, grid_z(batch * count));
   ProfScope prof(QTX_KERNEL_BLOCKOPS, 2.0 * sizeof(T) * n * n * (double)batch * count, s);
-  antiherm_kernel<T><<<grid, dim3(TILE, ROWS), 0, s>>>(n, batch, count, args, density, dens_stride, dens_off);
-  QTX_CHECK_LAUNCH();
-  return QTX_OK;
+  return launch_chained(antiherm_kernel<T>, grid, dim3(TILE, ROWS), 0, s, 1, n, batch, count, args, density,
+                        dens_stride, dens_off);
 }
 
 template <typename T>
@@ -408,10 +399,9 @@ int trace_t(int n, int64_t batch, int count, const MatRef* X, const MatRef* Y, c
     args.coef[k] = coef[k];
   }
   ProfScope prof(QTX_KERNEL_REDUCE, 2.0 * sizeof(T) * n * n * (double)batch * count, s);
-  cudaLaunchAttribute attr;
-  const cudaLaunchConfig_t cfg = cluster_config(batch, &attr, s);
-  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, trace_kernel<T>, n, batch, args, result, rstride, roff));
-  return QTX_OK;
+  const int S = reduce_split(batch);
+  return launch_chained(trace_kernel<T>, dim3((unsigned)(batch * S)), dim3(RT), 0, s, S, n, batch, args, result,
+                        rstride, roff);
 }
 
 template <typename TI, typename TO>

@@ -333,6 +333,7 @@ template <int OPA, int OPB, bool VEC>
 __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) cgemm_tc_kernel(const __grid_constant__ GroupArgs ga) {
   // 1024-byte alignment for the SWIZZLE_128B atoms.
   extern __shared__ __align__(1024) uint8_t smem[];
+  chain_begin();
   uint8_t* planes = smem;
   float2* tile = reinterpret_cast<float2*>(smem);  // epilogue tile [TM][S_LD], reuses the planes
   uint64_t* bar = reinterpret_cast<uint64_t*>(smem + PLANES_BYTES);
@@ -546,9 +547,7 @@ int launch_v(const GroupArgs& ga, cudaStream_t s) {
   const int64_t z = a.batch * ga.count;
   dim3 grid((a.N + TN - 1) / TN, (a.M + TM - 1) / TM, (unsigned)(z < 65535 ? z : 65535));
   ProfScope prof(QTX_KERNEL_CGEMM, 8.0 * a.M * a.N * (double)a.K * (double)z, s);
-  cgemm_tc_kernel<OPA, OPB, VEC><<<grid, THREADS, smem, s>>>(ga);
-  QTX_CHECK_LAUNCH();
-  return QTX_OK;
+  return launch_chained(cgemm_tc_kernel<OPA, OPB, VEC>, grid, dim3(THREADS), smem, s, 1, ga);
 }
 
 bool vec_ok(const MatRef& m) {

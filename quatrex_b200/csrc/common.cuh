@@ -72,6 +72,41 @@ const char* get_error();
     if (_s != QTX_OK) return _s;  \
   } while (0)
 
+// Programmatic dependent launch. A kernel started through launch_chained may be
+// scheduled while the kernel before it in the stream still runs its last CTAs;
+// chain_begin(), its first statement, lets the next one do the same and then
+// waits until everything before it has completed and is visible, so the order
+// of all memory accesses is that of a plain launch. It hides the launch gap of
+// chains of short kernels (an energy point of 16 blocks of 64 and 32 energies
+// 5.88 -> 5.65 ms, a selected solve of 6 blocks of about 28 1.00 -> 0.86 ms).
+#ifdef __CUDACC__
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory");
+  asm volatile("griddepcontrol.wait;\n" ::: "memory");
+}
+
+// cluster: CTAs per cluster along x (1: no cluster attribute).
+template <class... P, class... A>
+int launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, int cluster, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = (unsigned)cluster;
+  attr[1].val.clusterDim.y = 1;
+  attr[1].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = cluster > 1 ? 2 : 1;
+  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...));
+  return QTX_OK;
+}
+#endif
+
 // ---------------------------------------------------------------------------
 // Batched complex GEMM with a fused epilogue (zgemm.cu).
 //

@@ -240,6 +240,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) zgemm_kernel(const __gri
   constexpr int A_BYTES = stage_elems<BM, OPA == 0>() * 16;
   constexpr int B_BYTES = stage_elems<BN, OPB == 1>() * 16;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  chain_begin();
   const uint32_t as = smem_u32(smem_raw);
   const uint32_t bs = as + STAGES * A_BYTES;
 
@@ -371,9 +372,7 @@ int launch(const KernelArgs& args, cudaStream_t s) {
   const int64_t z = d.batch * args.count;
   dim3 grid((d.N + BN - 1) / BN, (d.M + BM - 1) / BM, (unsigned)(z < 65535 ? z : 65535));
   ProfScope prof(QTX_KERNEL_ZGEMM, 8.0 * d.M * d.N * (double)d.K * (double)z, s);
-  zgemm_kernel<OPA, OPB><<<grid, THREADS, smem, s>>>(args);
-  QTX_CHECK_LAUNCH();
-  return QTX_OK;
+  return launch_chained(zgemm_kernel<OPA, OPB>, grid, dim3(THREADS), smem, s, 1, args);
 }
 
 bool aligned16(const MatRef& m) { return (reinterpret_cast<uintptr_t>(m.p) & 15u) == 0; }

@@ -743,6 +743,7 @@ __global__ void __launch_bounds__(TH, 512 / TH) zinv3_kernel(int n, int64_t batc
   using S = Smem3;
   constexpr int NB = S::NB, WARPS3 = TH / 32;
   extern __shared__ __align__(16) unsigned char smem_raw[];
+  chain_begin();
   const int np = S::rows(n), YS = S::ys(n, csplit), XS = S::xs(n);
   z64* T = reinterpret_cast<z64*>(smem_raw);
   z64* Y = T + (size_t)np * NB;
@@ -947,8 +948,8 @@ int launch3(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* acti
   cudaLaunchAttribute attr;
   QTX_TRY((configure3<TH, RPL, RES>(n, batch, c, &cfg, &attr, s)));
   ProfScope prof(QTX_KERNEL_ZINV, 8.0 * (double)n * n * n * (double)batch, s);
-  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, zinv3_kernel<TH, RPL, RES>, n, batch, A, X, info, active, c));
-  return QTX_OK;
+  return launch_chained(zinv3_kernel<TH, RPL, RES>, cfg.gridDim, cfg.blockDim, cfg.dynamicSmemBytes, s, c, n, batch, A,
+                        X, info, active, c);
 }
 
 // Clusters of c CTAs of the column-split kernel that the GPU runs at once.

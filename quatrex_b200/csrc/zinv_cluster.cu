@@ -122,6 +122,7 @@ template <int C>
 __global__ void __launch_bounds__(CT, 1)
     zinv_cluster_kernel(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active,
                         const __grid_constant__ CUtensorMap tmap, int use_tma) {
+  chain_begin();
   cg::cluster_group cluster = cg::this_cluster();
   const int rank = (int)cluster.block_rank();
   const int64_t b = blockIdx.x / C;
@@ -376,21 +377,9 @@ int launch_cluster(int n, int64_t batch, MatRef A, MatRef X, int* info, const in
   CUtensorMap map;
   const int use_tma = make_map(&map, n, batch, A) ? 1 : 0;
   if (!use_tma) memset(&map, 0, sizeof(map));
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(batch * C), 1, 1);
-  cfg.blockDim = dim3(CT, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = s;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
   ProfScope prof(QTX_KERNEL_ZINV, 8.0 * (double)n * n * n * (double)batch, s);
-  QTX_CHECK_CUDA(cudaLaunchKernelEx(&cfg, zinv_cluster_kernel<C>, n, batch, A, X, info, active, map, use_tma));
-  return QTX_OK;
+  return launch_chained(zinv_cluster_kernel<C>, dim3((unsigned)(batch * C)), dim3(CT), smem, s, C, n, batch, A, X, info,
+                        active, map, use_tma);
 }
 
 }  // namespace
