@@ -160,9 +160,9 @@ int qtx_zinv_batched_ws(int n, int64_t batch, qtx_mat a, qtx_mat x, int* info, v
  * matrix that split its columns (n <= 512; C the largest of 2, 4, 8 leaving 32
  * columns per CTA). Automatic: the distributed-shared-memory cluster for
  * n <= 256 while batch x ceil(n / 32) is at most the SM count (half of it above
- * n = 128); else up to n = 512 the column split with the largest C for which
- * batch x C fits the SM count and every cluster is co-resident (C = 1 at full
- * batches, the matrix staying in shared memory up to n = 100); above n = 512
+ * n = 128); else up to n = 512 the column split with the largest C <= 8 (any
+ * number) for which batch x C fits the SM count and every cluster is
+ * co-resident (C = 1 at full batches, the matrix staying in shared memory up to n = 100); above n = 512
  * the multi-CTA path for batches up to half the SM count. All paths use the
  * same pivot rule; paths 1, 3 and 4 give bit-identical results up to n = 256,
  * 1 and 4 up to n = 512. A tuning and test knob; no reference counterpart. */

@@ -2,8 +2,8 @@
 // columns), shared by the one-CTA (zinv.cu) and the cluster
 // (zinv_cluster.cu) batched inverses.
 //
-// One thread holds one row of the panel for all of its columns, so a column
-// step touches shared memory only for the pivot search partials and the
+// LPR lanes (one or two) hold a row of the panel for all of its columns, lane h
+// of them columns h, h + LPR, ..., so a column step touches shared memory only for the pivot search partials and the
 // broadcast pivot row. Rows are not interchanged: each thread tracks the
 // position its row would have after LAPACK's interchanges. Per column k:
 //   pivot  p = argmax_{pos >= k} |Re| + |Im| of column k (lowest position on
@@ -20,13 +20,13 @@
 // words and a ballot, a slow path only if they tie) instead of five shuffle
 // rounds; the candidate's value travels with the search, so that every thread
 // forms 1 / x_pk itself while the pivot row is published; and the loop over the
-// columns is rolled. Cycles per column, factorization alone, at n = 64 / 256 /
-// 512: 1120 / 1455 / 2010 (two lanes to a row, five shuffle rounds and an
-// unrolled loop took about 3000 at n = 256). Measured beside it: two or four
-// lanes to a row with every warp publishing its candidate row and one barrier
-// 1130 / 2340 / - (a row written by one or two lanes costs as much as one
-// written by all), whole columns in a warp with the multipliers published
-// 1100 / 2440 / 4840; not inlined, 25 % slower in the inverse at n = 64.
+// columns is rolled. Cycles per column in the inverse at n = 64 / 128 / 256: with
+// one lane 1570 / 2020 / 2240, with two 1350 / 1660 / 2450 (half the row to
+// publish and to update, twice the warps to search), so two up to n = 128. (Two
+// lanes, five shuffle rounds and an unrolled loop took about 3000 at n = 256.)
+// Measured beside it, alone, at n = 64 / 256: one lane 1120 / 1455, every warp
+// publishing its candidate row ahead of a single barrier 1130 / 2340, whole
+// columns in a warp with the multipliers published 1100 / 2440.
 #pragma once
 
 #include "common.cuh"
@@ -111,18 +111,19 @@ __device__ __forceinline__ int gj_best_lane(unsigned long long key, int pos) {
   return __ffs(cand) - 1;
 }
 
-// Factors an n x nbp panel (nbp <= NB, n <= 512); the first ceil(n / 32) warps
-// of the CTA take part and the others return at once (named barrier 1).
+// Factors an n x nbp panel (nbp <= NB, n LPR <= 512); the first
+// ceil(n LPR / 32) warps of the CTA take part and the others return at once (named barrier 1).
 // load(r, c) / store(r, c, v): panel element access (r < n, c < nbp), the same
 // memory or not (a barrier separates loads and stores); moved(r, pos), once per
 // row after that barrier: row r ends at position pos. sing: shared int, set to
 // k + 1 at the first zero pivot if still 0.
-template <int NB, class Load, class Store, class Moved>
+template <int NB, int LPR, class Load, class Store, class Moved>
 __device__ __forceinline__ void gj_factor_panel(int n, int k0, int nbp, Load load, Store store, Moved moved,
                                                 int* sing) {
   __shared__ GjPanelSmem<NB> sm;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  const int W = (n + 31) >> 5;
+  constexpr int C = NB / LPR;
+  const int W = (n * LPR + 31) >> 5;
   if (warp >= W) return;
   const int bar_threads = W * 32;
   auto barrier = [&]() {
@@ -131,28 +132,32 @@ __device__ __forceinline__ void gj_factor_panel(int n, int k0, int nbp, Load loa
     else
       __syncwarp();
   };
-  const bool live = tid < n;
-  int pos = live ? tid : 0x7fffffff;
-  z64 v[NB];
+  const int r = tid / LPR, h = tid % LPR;
+  const bool live = r < n;
+  int pos = live ? r : 0x7fffffff;
+  z64 v[C];
 #pragma unroll
-  for (int c = 0; c < NB; ++c) v[c] = (live && c < nbp) ? load(tid, c) : make_double2(0.0, 0.0);
-  // The columns rotate through the registers: column k is always v[0], and
-  // the eliminated column enters at v[NB - 1]. The loop therefore stays
-  // rolled: unrolled over the columns its straight-line code (5 KB a column)
-  // is fetched anew for every panel and costs more than the arithmetic.
+  for (int i = 0; i < C; ++i)
+    v[i] = (live && h + i * LPR < nbp) ? load(r, h + i * LPR) : make_double2(0.0, 0.0);
 #pragma unroll 1
   for (int kk = 0; kk < nbp; ++kk) {
-    const int k = k0 + kk;
-    const bool mine = live && pos >= k;
+    const int k = k0 + kk, hk = kk % LPR;
+    z64 xk = v[0];
+    if (LPR > 1) {
+      const int src = (lane & ~(LPR - 1)) | hk;
+      xk.x = __shfl_sync(0xffffffffu, xk.x, src);
+      xk.y = __shfl_sync(0xffffffffu, xk.y, src);
+    }
+    const bool mine = live && pos >= k && h == hk;
     {
-      const double a = gj_abs1(v[0]);
+      const double a = gj_abs1(xk);
       // NaN compares false: such a row is never chosen
       const unsigned long long key = (mine && a >= 0.0) ? (unsigned long long)__double_as_longlong(a) + 1 : 0ull;
       const int tie = mine ? pos : 0x7fffffff;
       if (lane == gj_best_lane(key, tie)) {
         sm.key[warp] = key;
         sm.pos[warp] = tie;
-        sm.val[warp] = v[0];
+        sm.val[warp] = xk;
       }
     }
     barrier();
@@ -165,35 +170,51 @@ __device__ __forceinline__ void gj_factor_panel(int n, int k0, int nbp, Load loa
     z64* q = sm.q[kk & 1];
     if (piv) {
 #pragma unroll
-      for (int c = 1; c < NB; ++c) q[c] = v[c];
+      for (int i = 0; i < C; ++i) q[i * LPR + h] = v[i];
     }
     const z64 d = gj_recip(xp);
-    z64 m = gj_mul(v[0], d);
+    z64 m = gj_mul(xk, d);
     if (piv) {
-      // the scaled pivot row q / x_pk as 0 - (-1 / x_pk) q
       if (sm.key[wl] <= 1ull && *sing == 0) *sing = k + 1;
 #pragma unroll
-      for (int c = 1; c < NB; ++c) v[c] = make_double2(0.0, 0.0);
+      for (int i = 0; i < C; ++i) v[i] = make_double2(0.0, 0.0);  // q / x_pk as 0 - (-1 / x_pk) q
       m = make_double2(-d.x, -d.y);
       pos = k;
     } else if (pos == k) {
       pos = p;
     }
     barrier();
+    // The columns rotate through the registers (every LPR steps): column k is
+    // always in v[0]. The loop therefore stays rolled: unrolled over the columns
+    // its straight-line code (5 KB a column) is fetched anew for every panel and
+    // costs more than the arithmetic.
+    if (LPR == 1) {
 #pragma unroll
-    for (int c = 1; c < NB; ++c) {
-      v[c - 1] = gj_eliminate(v[c], m, q[c]);
-      if (c % 5 == 0) asm volatile("" ::: "memory");  // bounds the loads in flight (registers)
+      for (int i = 1; i < C; ++i) {
+        v[i - 1] = gj_eliminate(v[i], m, q[i]);
+        if (i % 5 == 0) asm volatile("" ::: "memory");  // bounds the loads in flight (registers)
+      }
+      v[C - 1] = make_double2(-m.x, -m.y);
+    } else {
+#pragma unroll
+      for (int i = 0; i < C; ++i) v[i] = gj_eliminate(v[i], m, q[i * LPR + h]);
+      if (h == hk) v[0] = make_double2(-m.x, -m.y);
+      if (hk == LPR - 1) {
+        const z64 f = v[0];
+#pragma unroll
+        for (int i = 0; i + 1 < C; ++i) v[i] = v[i + 1];
+        v[C - 1] = f;
+      }
     }
-    v[NB - 1] = make_double2(-m.x, -m.y);
   }
   barrier();  // every load of the panel (and of the last pivot row) is done
   if (live) {
-    moved(tid, pos);
+    if (h == 0) moved(r, pos);
 #pragma unroll
-    for (int c = 0; c < NB; ++c) {
-      const int col = c + nbp < NB ? c + nbp : c + nbp - NB;  // after nbp rotations
-      if (col < nbp) store(pos, col, v[c]);
+    for (int i = 0; i < C; ++i) {
+      const int g = i + nbp / LPR;
+      const int col = h + LPR * (g < C ? g : g - C);  // after nbp / LPR rotations
+      if (col < nbp) store(pos, col, v[i]);
     }
   }
 }

@@ -23,6 +23,8 @@
 // Total work n^3 complex multiply-adds = 8 n^3 real flops.
 #include <cooperative_groups.h>
 
+#include <algorithm>
+
 #include "common.cuh"
 #include "gj_panel.cuh"
 
@@ -783,7 +785,7 @@ __global__ void __launch_bounds__(TH, 512 / TH) zinv3_kernel(int n, int64_t batc
     for (int k0 = 0; k0 < n; k0 += NB) {
       const int nbp = min(NB, n - k0), kt = k0 / NB;
       // 1. Factor the panel.
-      gj_factor_panel<NB>(
+      gj_factor_panel<NB, RPL <= 4 ? 2 : 1>(
           n, k0, nbp,
           [=](int r, int c) { return RES ? x[r * ldx + k0 + c] : __ldcg(&x[r * ldx + k0 + c]); },
           [=](int r, int c, z64 v) { T[tix(r, c)] = v; },
@@ -813,76 +815,82 @@ __global__ void __launch_bounds__(TH, 512 / TH) zinv3_kernel(int n, int64_t batc
         }
       }
       __syncthreads();
-      // 3./4. Update of one 16 x 16 tile at row slice mt, local columns j0.
-      z64 t0[NB / 4], t1[NB / 4];  // this slice's rows of T, DMMA fragments
-      auto load_t = [&](int mt) {
-#pragma unroll
-        for (int k4 = 0; k4 < NB; k4 += 4) {
-          t0[k4 / 4] = T[tix(mt * 16 + g, k4 + tq)];
-          t1[k4 / 4] = T[tix(mt * 16 + g + 8, k4 + tq)];
-        }
-      };
-      auto update = [&](int mt, int j0, const z64* s0, const z64* s1) {
-        double cre[2][4], cim[2][4];
-        const int cl = j0 + 2 * tq;
+      // 3./4. Tiles of 16 x 16 outside the panel's columns, dealt evenly in
+      // row-slice order. A tile's elements are loaded (the accumulators) while
+      // the one before is multiplied.
+      const int pt = pin ? (k0 - c_lo) / 16 : ntiles, nt = ntiles - (pin ? 1 : 0);
+      auto load_c = [&](int mt, int j0, double(&re)[2][4], double(&im)[2][4]) {
+        const int ra = mt * 16 + g, cl = j0 + 2 * tq;
+        const z64* s0 = ra < n ? x + srcrow[ra] * ldx + c_lo + cl : nullptr;
+        const z64* s1 = ra + 8 < n ? x + srcrow[ra + 8] * ldx + c_lo + cl : nullptr;
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const z64* sr = (q >> 1) ? s1 : s0;
-            const int cc = cl + j * 8 + (q & 1);
-            const z64 v = (sr != nullptr && cc < cw) ? sr[cc] : make_double2(0.0, 0.0);
-            cre[j][q] = v.x;
-            cim[j][q] = v.y;
+            const int o = j * 8 + (q & 1);
+            const z64 v = (sr != nullptr && cl + o < cw) ? sr[o] : make_double2(0.0, 0.0);
+            re[j][q] = v.x;
+            im[j][q] = v.y;
           }
+      };
+      auto update = [&](int mt, int j0, double(&re)[2][4], double(&im)[2][4]) {
 #pragma unroll
         for (int k4 = 0; k4 < NB; k4 += 4) {
-          const z64 v0 = t0[k4 / 4], v1 = t1[k4 / 4];
+          const z64 v0 = T[tix(mt * 16 + g, k4 + tq)], v1 = T[tix(mt * 16 + g + 8, k4 + tq)];
           z64 y[2];
 #pragma unroll
           for (int j = 0; j < 2; ++j) y[j] = Y[(k4 + tq) * YS + j0 + j * 8 + g];
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            mma_f64(cre[j], v0.x, v1.x, y[j].x);
-            mma_f64(cim[j], v0.x, v1.x, y[j].y);
+            mma_f64(re[j], v0.x, v1.x, y[j].x);
+            mma_f64(im[j], v0.x, v1.x, y[j].y);
           }
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
-            mma_f64(cre[j], -v0.y, -v1.y, y[j].y);
-            mma_f64(cim[j], v0.y, v1.y, y[j].x);
+            mma_f64(re[j], -v0.y, -v1.y, y[j].y);
+            mma_f64(im[j], v0.y, v1.y, y[j].x);
           }
         }
+        const int cl = j0 + 2 * tq;
 #pragma unroll
         for (int j = 0; j < 2; ++j)
 #pragma unroll
           for (int q = 0; q < 4; ++q) {
             const int r = mt * 16 + g + ((q >> 1) << 3), cc = cl + j * 8 + (q & 1);
-            if (r < n && cc < cw) x[r * ldx + c_lo + cc] = make_double2(cre[j][q], cim[j][q]);
+            if (r < n && cc < cw) x[r * ldx + c_lo + cc] = make_double2(re[j][q], im[j][q]);
           }
       };
-      // Tiles outside the panel's columns, dealt evenly in row-slice order.
-      const int pt = pin ? (k0 - c_lo) / 16 : ntiles, nt = ntiles - (pin ? 1 : 0);
       const int total = (mtiles - 1) * nt;
       const int u0 = (int)((int64_t)total * warp / WARPS3), u1 = (int)((int64_t)total * (warp + 1) / WARPS3);
-      int last = -1;
-      const z64 *s0 = nullptr, *s1 = nullptr;
-      for (int u = u0; u < u1; ++u) {
-        int mt = u / nt, jt = u % nt;
-        if (mt >= kt) ++mt;
-        if (jt >= pt) ++jt;
-        if (mt != last) {
-          last = mt;
-          load_t(mt);
-          const int ra = mt * 16 + g;
-          s0 = ra < n ? x + srcrow[ra] * ldx + c_lo : nullptr;
-          s1 = ra + 8 < n ? x + srcrow[ra + 8] * ldx + c_lo : nullptr;
+      if (u0 < u1) {
+        int m = u0 / nt, j = u0 % nt;
+        double re[2][4], im[2][4], nre[2][4], nim[2][4];
+        auto slice = [&](int v) { return v >= kt ? v + 1 : v; };
+        auto column = [&](int v) { return (v >= pt ? v + 1 : v) * 16; };
+        load_c(slice(m), column(j), re, im);
+#pragma unroll 1
+        for (int u = u0; u < u1; ++u) {
+          const int mt = slice(m), j0 = column(j);
+          if (++j == nt) {
+            j = 0;
+            ++m;
+          }
+          if (u + 1 < u1) load_c(slice(m), column(j), nre, nim);
+          update(mt, j0, re, im);
+#pragma unroll
+          for (int jj = 0; jj < 2; ++jj)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              re[jj][q] = nre[jj][q];
+              im[jj][q] = nim[jj][q];
+            }
         }
-        update(mt, jt * 16, s0, s1);
       }
       __syncthreads();
-      if (warp < nt) {
-        load_t(kt);
-        for (int u = warp; u < nt; u += WARPS3) update(kt, (u >= pt ? u + 1 : u) * 16, nullptr, nullptr);
+      for (int u = warp; u < nt; u += WARPS3) {
+        double re[2][4] = {}, im[2][4] = {};
+        update(kt, (u >= pt ? u + 1 : u) * 16, re, im);
       }
       __syncthreads();
       cluster_sync();
@@ -983,23 +991,25 @@ int active_clusters(int n, int c) {
 constexpr size_t kMaxSmem3 = 227 * 1024 - sizeof(GjPanelSmem<16>) - 64;  // beside the static shared memory
 bool fits_resident(int n) { return n <= 128 && Smem3::bytes(n, 1, true) <= kMaxSmem3; }
 
-// Column split of the n <= 512 kernel: the largest C in {1, 2, 4, 8} with
-// batch x C within the SM count, at least 32 columns per CTA, and all batch
-// clusters co-resident. Inverse path 4 forces the largest C the block size
-// allows; 2 is the least where one CTA's pivot rows and transform do not fit.
+// Column split of the n <= 512 kernel: the largest C <= 8 with batch x C within
+// the SM count, at least 32 columns per CTA, and all batch clusters
+// co-resident; at least two where one CTA's pivot rows and transform do not fit.
+// (Powers of two alone left 64 of 148 SMs idle at n = 512, batch 42: 5.0 ms
+// against 3.6 with C = 3.) Inverse path 4 forces the largest power of two
+// that the block size allows.
 int column_split(int n, int64_t batch) {
   const int path = inverse_path();
   int least = 1;
-  while (Smem3::bytes(n, least, false) > kMaxSmem3) least *= 2;
+  while (Smem3::bytes(n, least, false) > kMaxSmem3) ++least;
   if (path != 0 && path != 4) return least;
-  int cmax = 1;
-  while (cmax < 8 && n / (2 * cmax) >= 32) cmax *= 2;
-  if (path == 4) return cmax > least ? cmax : least;
-  const int sms = num_sms();
-  int c = least;
-  while (c < cmax && batch * (2 * c) <= sms) c *= 2;
-  while (c > least && active_clusters(n, c) < batch) c /= 2;
-  return c;
+  if (path == 4) {
+    int c = 1;
+    while (c < 8 && n / (2 * c) >= 32) c *= 2;
+    return c > least ? c : least;
+  }
+  int c = (int)std::min<int64_t>(std::min(8, n / 32), num_sms() / std::max<int64_t>(batch, 1));
+  while (c > least && active_clusters(n, c) < batch) --c;
+  return c > least ? c : least;
 }
 
 int launch_split(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s) {

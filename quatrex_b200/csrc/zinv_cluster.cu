@@ -199,7 +199,7 @@ __global__ void __launch_bounds__(CT, 1)
     const uint32_t tbytes = (uint32_t)(2 * chunk * sizeof(z64)) + (uint32_t)npad * sizeof(int);
 
     if (own) {
-      gj_factor_panel<CNB>(
+      gj_factor_panel<CNB, C <= 4 ? 2 : 1>(
           n, k0, nbp, [=](int r, int c) { return Xs[xoff(npad, r, kl + c)]; },
           [=](int r, int c, z64 v) { Xs[xoff(npad, r, kl + c)] = v; },
           [=](int r, int pos) { srcrow[pos] = r; }, &s_sing);
