@@ -167,82 +167,97 @@ __device__ __forceinline__ void b_task(int t, int& row, int& chunk) {
   }
 }
 
-// Global -> registers for one K block (all loads issued back to back). With
-// VEC (operands 16-byte aligned, even leading dimensions) the K-contiguous
-// operands are read two complex numbers per 16-byte load.
+// A K-contiguous operand with VEC (16-byte aligned, even leading dimension) is
+// read two complex numbers per load, pair t of (row, pair of k): 16 lanes read a
+// row's 256 bytes of the K block. Four k per thread in two such loads, a gap of
+// 16 bytes between lanes, took 16 wavefronts a load instead of 4, and the L1 /
+// shared data pipe is what bounds this kernel (loads and stores 154 k wavefronts
+// and the MMAs' operand reads 98 k in 253 k cycles; tensor pipe 39 %): 148
+// products of 256^3 NN 148 -> 134 us, NT 157 -> 144 us. With op(A) in TMEM,
+// which spares the pipe those stores and reads, the chain of fetch, split and
+// MMA bounds it instead: 140 and 149 us (143 and 169 us with two K blocks of 16
+// in flight).
+__device__ __forceinline__ void pair_task(int t, int& row, int& pair) {
+  row = t >> 4;
+  pair = t & 15;
+}
+
+// Pair `pair` of k of row gr (rows of X are K-contiguous); zeros outside.
+__device__ __forceinline__ float4 load_pair(const c32* X, int64_t ld, int gr, int rows, int gk, int K) {
+  float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+  if (gr < rows && gk + 1 < K) {
+    v = *reinterpret_cast<const float4*>(X + (int64_t)gr * ld + gk);
+  } else if (gr < rows && gk < K) {
+    const float2 w = X[(int64_t)gr * ld + gk];
+    v = make_float4(w.x, w.y, 0.f, 0.f);
+  }
+  return v;
+}
+
+// Global -> registers for one K block (all loads issued back to back).
 template <int OPA, int OPB, bool VEC>
 __device__ __forceinline__ void load_regs(const Args& a, const c32* Ag, const c32* Bg, Regs& R, int m0,
                                           int n0, int k0, int tid) {
+  if (OPA == 0 && VEC) {
 #pragma unroll
-  for (int i = 0; i < A_TASKS; ++i) {
-    int row, chunk;
-    a_task<OPA>(tid + i * THREADS, row, chunk);
-    const int gr = m0 + row;
-    if (OPA == 0 && VEC) {
-#pragma unroll
-      for (int e = 0; e < 4; e += 2) {
-        const int gk = k0 + chunk * 4 + e;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (gr < a.M && gk + 1 < a.K) {
-          v = *reinterpret_cast<const float4*>(Ag + (int64_t)gr * a.A.ld + gk);
-        } else if (gr < a.M && gk < a.K) {
-          const float2 w = Ag[(int64_t)gr * a.A.ld + gk];
-          v = make_float4(w.x, w.y, 0.f, 0.f);
-        }
-        R.a[i][e] = make_float2(v.x, v.y);
-        R.a[i][e + 1] = make_float2(v.z, v.w);
-      }
-      continue;
+    for (int i = 0; i < 2 * A_TASKS; ++i) {
+      int row, pair;
+      pair_task(tid + i * THREADS, row, pair);
+      const float4 v = load_pair(Ag, a.A.ld, m0 + row, a.M, k0 + 2 * pair, a.K);
+      R.a[i >> 1][(i & 1) * 2] = make_float2(v.x, v.y);
+      R.a[i >> 1][(i & 1) * 2 + 1] = make_float2(v.z, v.w);
     }
+  } else {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int gk = k0 + chunk * 4 + e;
-      float2 v = make_float2(0.f, 0.f);
-      if (gr < a.M && gk < a.K) {
-        if (OPA == 0) {
-          v = Ag[(int64_t)gr * a.A.ld + gk];
-        } else {
-          v = Ag[(int64_t)gk * a.A.ld + gr];
-          v.y = -v.y;
+    for (int i = 0; i < A_TASKS; ++i) {
+      int row, chunk;
+      a_task<OPA>(tid + i * THREADS, row, chunk);
+      const int gr = m0 + row;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int gk = k0 + chunk * 4 + e;
+        float2 v = make_float2(0.f, 0.f);
+        if (gr < a.M && gk < a.K) {
+          if (OPA == 0) {
+            v = Ag[(int64_t)gr * a.A.ld + gk];
+          } else {
+            v = Ag[(int64_t)gk * a.A.ld + gr];
+            v.y = -v.y;
+          }
         }
+        R.a[i][e] = v;
       }
-      R.a[i][e] = v;
     }
   }
+  if (OPB == 1 && VEC) {
 #pragma unroll
-  for (int i = 0; i < B_TASKS; ++i) {
-    int row, chunk;
-    b_task<OPB>(tid + i * THREADS, row, chunk);
-    const int gn = n0 + row;
-    if (OPB == 1 && VEC) {
-#pragma unroll
-      for (int e = 0; e < 4; e += 2) {
-        const int gk = k0 + chunk * 4 + e;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (gn < a.N && gk + 1 < a.K) {
-          v = *reinterpret_cast<const float4*>(Bg + (int64_t)gn * a.B.ld + gk);
-        } else if (gn < a.N && gk < a.K) {
-          const float2 w = Bg[(int64_t)gn * a.B.ld + gk];
-          v = make_float4(w.x, w.y, 0.f, 0.f);
-        }
-        R.b[i][e] = make_float2(v.x, -v.y);
-        R.b[i][e + 1] = make_float2(v.z, -v.w);
-      }
-      continue;
+    for (int i = 0; i < 2 * B_TASKS; ++i) {
+      int row, pair;
+      pair_task(tid + i * THREADS, row, pair);
+      const float4 v = load_pair(Bg, a.B.ld, n0 + row, a.N, k0 + 2 * pair, a.K);
+      R.b[i >> 1][(i & 1) * 2] = make_float2(v.x, -v.y);
+      R.b[i >> 1][(i & 1) * 2 + 1] = make_float2(v.z, -v.w);
     }
+  } else {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int gk = k0 + chunk * 4 + e;
-      float2 v = make_float2(0.f, 0.f);
-      if (gn < a.N && gk < a.K) {
-        if (OPB == 0) {
-          v = Bg[(int64_t)gk * a.B.ld + gn];
-        } else {
-          v = Bg[(int64_t)gn * a.B.ld + gk];
-          v.y = -v.y;
+    for (int i = 0; i < B_TASKS; ++i) {
+      int row, chunk;
+      b_task<OPB>(tid + i * THREADS, row, chunk);
+      const int gn = n0 + row;
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const int gk = k0 + chunk * 4 + e;
+        float2 v = make_float2(0.f, 0.f);
+        if (gn < a.N && gk < a.K) {
+          if (OPB == 0) {
+            v = Bg[(int64_t)gk * a.B.ld + gn];
+          } else {
+            v = Bg[(int64_t)gn * a.B.ld + gk];
+            v.y = -v.y;
+          }
         }
+        R.b[i][e] = v;
       }
-      R.b[i][e] = v;
     }
   }
 }
@@ -264,35 +279,79 @@ __device__ __forceinline__ void split4(const float2 (&v)[4], float4& hr, float4&
 
 __device__ __forceinline__ float4 neg4(float4 v) { return make_float4(-v.x, -v.y, -v.z, -v.w); }
 
+// hi and lo of two values.
+__device__ __forceinline__ void split2(float x, float y, float2& h, float2& l) {
+  h = make_float2(tf32_trunc(x), tf32_trunc(y));
+  l = make_float2(tf32_trunc(x - h.x), tf32_trunc(y - h.y));
+}
+
+__device__ __forceinline__ float2 neg2(float2 v) { return make_float2(-v.x, -v.y); }
+
 // Registers -> the split planes (SWIZZLE_128B K-major).
-template <int OPA, int OPB>
+template <int OPA, int OPB, bool VEC>
 __device__ __forceinline__ void store_planes(const Regs& R, uint8_t* planes, int tid) {
   uint8_t* pb = planes + 4 * PLANE_A;
+  if (OPA == 0 && VEC) {
 #pragma unroll
-  for (int i = 0; i < A_TASKS; ++i) {
-    int row, chunk;
-    a_task<OPA>(tid + i * THREADS, row, chunk);
-    float4 hr, lr, hi, li;
-    split4(R.a[i], hr, lr, hi, li);
-    const uint32_t off = sw128_offset(row, chunk);
-    *reinterpret_cast<float4*>(planes + off) = hr;
-    *reinterpret_cast<float4*>(planes + PLANE_A + off) = lr;
-    *reinterpret_cast<float4*>(planes + 2 * PLANE_A + off) = hi;
-    *reinterpret_cast<float4*>(planes + 3 * PLANE_A + off) = li;
+    for (int i = 0; i < 2 * A_TASKS; ++i) {
+      int row, pair;
+      pair_task(tid + i * THREADS, row, pair);
+      const float2 u = R.a[i >> 1][(i & 1) * 2], v = R.a[i >> 1][(i & 1) * 2 + 1];
+      float2 hr, lr, hi, li;
+      split2(u.x, v.x, hr, lr);
+      split2(u.y, v.y, hi, li);
+      const uint32_t off = sw128_offset(row, pair >> 1) + 8 * (pair & 1);
+      *reinterpret_cast<float2*>(planes + off) = hr;
+      *reinterpret_cast<float2*>(planes + PLANE_A + off) = lr;
+      *reinterpret_cast<float2*>(planes + 2 * PLANE_A + off) = hi;
+      *reinterpret_cast<float2*>(planes + 3 * PLANE_A + off) = li;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < A_TASKS; ++i) {
+      int row, chunk;
+      a_task<OPA>(tid + i * THREADS, row, chunk);
+      float4 hr, lr, hi, li;
+      split4(R.a[i], hr, lr, hi, li);
+      const uint32_t off = sw128_offset(row, chunk);
+      *reinterpret_cast<float4*>(planes + off) = hr;
+      *reinterpret_cast<float4*>(planes + PLANE_A + off) = lr;
+      *reinterpret_cast<float4*>(planes + 2 * PLANE_A + off) = hi;
+      *reinterpret_cast<float4*>(planes + 3 * PLANE_A + off) = li;
+    }
   }
+  if (OPB == 1 && VEC) {
 #pragma unroll
-  for (int i = 0; i < B_TASKS; ++i) {
-    int row, chunk;
-    b_task<OPB>(tid + i * THREADS, row, chunk);
-    float4 hr, lr, hi, li;
-    split4(R.b[i], hr, lr, hi, li);
-    const uint32_t off = sw128_offset(row, chunk);
-    *reinterpret_cast<float4*>(pb + off) = neg4(hi);
-    *reinterpret_cast<float4*>(pb + PLANE_B + off) = hr;
-    *reinterpret_cast<float4*>(pb + 2 * PLANE_B + off) = hi;
-    *reinterpret_cast<float4*>(pb + 3 * PLANE_B + off) = neg4(li);
-    *reinterpret_cast<float4*>(pb + 4 * PLANE_B + off) = lr;
-    *reinterpret_cast<float4*>(pb + 5 * PLANE_B + off) = li;
+    for (int i = 0; i < 2 * B_TASKS; ++i) {
+      int row, pair;
+      pair_task(tid + i * THREADS, row, pair);
+      const float2 u = R.b[i >> 1][(i & 1) * 2], v = R.b[i >> 1][(i & 1) * 2 + 1];
+      float2 hr, lr, hi, li;
+      split2(u.x, v.x, hr, lr);
+      split2(u.y, v.y, hi, li);
+      const uint32_t off = sw128_offset(row, pair >> 1) + 8 * (pair & 1);
+      *reinterpret_cast<float2*>(pb + off) = neg2(hi);
+      *reinterpret_cast<float2*>(pb + PLANE_B + off) = hr;
+      *reinterpret_cast<float2*>(pb + 2 * PLANE_B + off) = hi;
+      *reinterpret_cast<float2*>(pb + 3 * PLANE_B + off) = neg2(li);
+      *reinterpret_cast<float2*>(pb + 4 * PLANE_B + off) = lr;
+      *reinterpret_cast<float2*>(pb + 5 * PLANE_B + off) = li;
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < B_TASKS; ++i) {
+      int row, chunk;
+      b_task<OPB>(tid + i * THREADS, row, chunk);
+      float4 hr, lr, hi, li;
+      split4(R.b[i], hr, lr, hi, li);
+      const uint32_t off = sw128_offset(row, chunk);
+      *reinterpret_cast<float4*>(pb + off) = neg4(hi);
+      *reinterpret_cast<float4*>(pb + PLANE_B + off) = hr;
+      *reinterpret_cast<float4*>(pb + 2 * PLANE_B + off) = hi;
+      *reinterpret_cast<float4*>(pb + 3 * PLANE_B + off) = neg4(li);
+      *reinterpret_cast<float4*>(pb + 4 * PLANE_B + off) = lr;
+      *reinterpret_cast<float4*>(pb + 5 * PLANE_B + off) = li;
+    }
   }
 }
 
@@ -373,7 +432,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) cgemm_tc_kernel(const __
     const c32* Bg = at<const c32>(a.B, b);
     if (KB > 0) {
       load_regs<OPA, OPB, VEC>(a, Ag, Bg, R, m0, n0, 0, tid);
-      store_planes<OPA, OPB>(R, planes, tid);
+      store_planes<OPA, OPB, VEC>(R, planes, tid);
       fence_async_smem();
       __syncthreads();
     }
@@ -394,7 +453,7 @@ __global__ void __launch_bounds__(THREADS, CTAS_PER_SM) cgemm_tc_kernel(const __
       phase ^= 1u;
       ok = __syncthreads_and(ok);
       if (more && ok) {
-        store_planes<OPA, OPB>(R, planes, tid);
+        store_planes<OPA, OPB, VEC>(R, planes, tid);
         fence_async_smem();
       }
       if (!__syncthreads_and(ok)) {
