@@ -698,8 +698,9 @@ int launch2(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* acti
 //   1. every CTA factors the panel itself (gj_panel.cuh; the same arithmetic on
 //      the same data, so the same transform and pivots) -- no broadcast;
 //      rows are not interchanged, the factorization only says where they go;
-//   2. the pivot rows Y of this CTA's columns are staged, and the owner of the
-//      panel's columns writes the transform T there;
+//   2. the pivot rows Y of this CTA's columns are staged, and, once every CTA of
+//      the cluster has loaded the panel (a split cluster barrier), the owner of
+//      its columns writes the transform T there;
 //   3. all row slices but the pivots' own are updated, X[r, J] <- X[src(r), J]
 //      + T[r, :] Y[:, J] (DMMA): src(r) is r, or the row of K that LAPACK's
 //      interchanges would have moved to r, so the interchange costs no pass of
@@ -795,6 +796,12 @@ __global__ void __launch_bounds__(TH, 512 / TH) zinv3_kernel(int n, int64_t batc
           },
           &s_sing);
       cur ^= 1;
+      // This CTA's loads of the panel are done. The owner may store the
+      // transform over X[:, K] only when that holds for every CTA of the
+      // cluster, so all arrive here and wait ahead of that store; the pivot rows
+      // are staged meanwhile. (All CTAs factor in step, so the wait
+      // is short: 256 x 18 530 -> 536 us, 384 x 37 1.68 -> 1.70 ms, 512 x 21 2.24 -> 2.25.)
+      if (!RES && csplit > 1) cg::this_cluster().barrier_arrive();
       __syncthreads();
       // 2. Pivot rows of this CTA's other columns; the transform into X[:, K].
       const bool pin = k0 >= c_lo && k0 < c_hi;
@@ -805,6 +812,7 @@ __global__ void __launch_bounds__(TH, 512 / TH) zinv3_kernel(int n, int64_t batc
         for (int j = lane; j < YS - 2; j += 32)
           Y[kk * YS + j] = (xr != nullptr && j < cw && (j < p0 || j >= p1)) ? xr[j] : make_double2(0.0, 0.0);
       }
+      if (!RES && csplit > 1) cg::this_cluster().barrier_wait();
       {
         const int c = tid % NB;
         if (c >= nbp) {  // columns of T that the factorization left unwritten

@@ -112,3 +112,33 @@ def test_split_singular_report_and_automatic_choice(cuda_device, path):
         ok = np.arange(B) != 2
         np.testing.assert_array_equal(outs[mode][ok], outs[1][ok])
     assert infos[1][2] == 78 and (infos[1][np.arange(B) != 2] == 0).all()
+
+
+@pytest.mark.parametrize("n,batch", [(225, 21), (226, 18), (255, 18), (256, 24), (257, 18), (257, 29), (272, 37), (385, 37),
+                                     (386, 49), (399, 21), (400, 74), (512, 18)])
+def test_every_split_beside_other_work(cuda_device, path, n, batch):
+    """Automatic splits of 2 to 8 CTAs with last panels of 1, 2, 15 and 16
+    columns, while products on another stream load the memory system: the bits
+    of the single-CTA path (two CTAs at 512), several times over. (The order of
+    the CTAs' accesses itself is checked in test_column_split_order.py.)"""
+    rng = np.random.default_rng(n)
+    A = torch.from_numpy(_rand(rng, batch, n, n)).to(cuda_device)
+    w = torch.from_numpy(_rand(rng, 32, 128, 128)).to(cuda_device)
+    out = torch.empty_like(w)
+    path(1)
+    ref = torch.empty_like(A)
+    assert not _inv(mat(A), mat(ref), n, batch, cuda_device).any()
+    path(0)
+    side = torch.cuda.Stream()
+    lib = _native.load()
+    x = torch.empty_like(A)
+    info = torch.zeros(batch, dtype=torch.int32, device=cuda_device)
+    torch.cuda.synchronize()
+    for _ in range(4):
+        x.fill_(float("nan"))
+        for _ in range(24):
+            _native.check(lib.qtx_zgemm_batched(128, 128, 128, 32, 1.0, 0.0, mat(w), 0, mat(w), 0, 0.0, 0.0,
+                                                _native.NULL_MAT, 0, mat(out), ctypes.c_void_p(side.cuda_stream)))
+        _native.check(lib.qtx_zinv_batched(n, batch, mat(A), mat(x), info.data_ptr(), _stream()))
+        torch.cuda.synchronize()
+        assert torch.equal(x, ref) and not info.any()
