@@ -72,6 +72,22 @@ const char* get_error();
     if (_s != QTX_OK) return _s;  \
   } while (0)
 
+// Dynamic shared memory a CTA may ask for: 227 KB less 1 KB for a kernel's
+// static arrays.
+constexpr size_t kMaxDynamicSmem = 226 * 1024;
+
+#ifdef __CUDACC__
+// Allows `kernel` to be launched with up to kMaxDynamicSmem bytes. The limit is
+// one attribute per kernel for all host threads, so it is always set to the
+// same value, never to the bytes of one call: another thread's smaller call
+// between this and the launch would make the launch fail.
+template <class... P>
+int allow_dynamic_smem(void (*kernel)(P...)) {
+  QTX_CHECK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDynamicSmem));
+  return QTX_OK;
+}
+#endif
+
 // Programmatic dependent launch. A kernel started through launch_chained may be
 // scheduled while the kernel before it in the stream still runs its last CTAs;
 // chain_begin(), its first statement, lets the next one do the same and then

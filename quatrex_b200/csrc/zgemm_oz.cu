@@ -840,7 +840,7 @@ int run_split(const MatRef& X, int rows, int K, int conj, bool isb, bool strided
     const size_t smem = (size_t)STRIP_ROWS * strip_len(g.Kc) * sizeof(double2);
     dim3 grid(rows_p / STRIP_ROWS, (unsigned)bc);
     auto launch = [&](auto kern) -> int {
-      QTX_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+      QTX_TRY(allow_dynamic_smem(kern));
       kern<<<grid, THREADS, smem, s>>>(a);
       return QTX_OK;
     };

@@ -348,12 +348,11 @@ __global__ void __launch_bounds__(THREADS, 1) zinv_kernel(int n, int64_t batch, 
 template <int NB>
 int launch(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s) {
   const size_t smem = Smem<NB>::bytes(n);
-  if (smem > 227 * 1024) {
+  if (smem > kMaxDynamicSmem) {
     set_error("zinv: block size too large for the shared-memory panel");
     return QTX_ERR_UNSUPPORTED;
   }
-  QTX_CHECK_CUDA(
-      cudaFuncSetAttribute(zinv_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  QTX_TRY(allow_dynamic_smem(zinv_kernel<NB>));
   const unsigned grid = (unsigned)(batch < 1048576 ? batch : 1048576);
   ProfScope prof(QTX_KERNEL_ZINV, 8.0 * (double)n * n * n * (double)batch, s);
   zinv_kernel<NB><<<grid, THREADS, smem, s>>>(n, batch, A, X, info, active);
@@ -678,12 +677,11 @@ __global__ void __launch_bounds__(T2, 1) zinv2_kernel(int n, int64_t batch, MatR
 template <int NB>
 int launch2(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s) {
   const size_t smem = Smem2<NB>::bytes(n);
-  if (smem > 227 * 1024) {
+  if (smem > kMaxDynamicSmem) {
     set_error("zinv: block size too large for the shared-memory panel");
     return QTX_ERR_UNSUPPORTED;
   }
-  QTX_CHECK_CUDA(
-      cudaFuncSetAttribute(zinv2_kernel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  QTX_TRY(allow_dynamic_smem(zinv2_kernel<NB>));
   const unsigned grid = (unsigned)(batch < 131072 ? batch : 131072);
   ProfScope prof(QTX_KERNEL_ZINV, 8.0 * (double)n * n * n * (double)batch, s);
   zinv2_kernel<NB><<<grid, T2, smem, s>>>(n, batch, A, X, info, active);
@@ -941,8 +939,7 @@ __global__ void __launch_bounds__(TH, 512 / TH) zinv3_kernel(int n, int64_t batc
 template <int TH, int RPL, bool RES>
 int configure3(int n, int64_t batch, int c, cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, cudaStream_t s) {
   const size_t smem = Smem3::bytes(n, c, RES);
-  QTX_CHECK_CUDA(cudaFuncSetAttribute(zinv3_kernel<TH, RPL, RES>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+  QTX_TRY((allow_dynamic_smem(zinv3_kernel<TH, RPL, RES>)));
   const int64_t mats = batch < 131072 ? batch : 131072;
   *cfg = {};
   cfg->gridDim = dim3((unsigned)(mats * c), 1, 1);
@@ -996,8 +993,8 @@ int active_clusters(int n, int c) {
   return nc;
 }
 
-constexpr size_t kMaxSmem3 = 227 * 1024 - sizeof(GjPanelSmem<16>) - 64;  // beside the static shared memory
-bool fits_resident(int n) { return n <= 128 && Smem3::bytes(n, 1, true) <= kMaxSmem3; }
+static_assert(sizeof(GjPanelSmem<16>) + 64 <= 1024, "static shared memory beside kMaxDynamicSmem");
+bool fits_resident(int n) { return n <= 128 && Smem3::bytes(n, 1, true) <= kMaxDynamicSmem; }
 
 // Column split of the n <= 512 kernel: the largest C <= 8 with batch x C within
 // the SM count, at least 32 columns per CTA, and all batch clusters
@@ -1008,7 +1005,7 @@ bool fits_resident(int n) { return n <= 128 && Smem3::bytes(n, 1, true) <= kMaxS
 int column_split(int n, int64_t batch) {
   const int path = inverse_path();
   int least = 1;
-  while (Smem3::bytes(n, least, false) > kMaxSmem3) ++least;
+  while (Smem3::bytes(n, least, false) > kMaxDynamicSmem) ++least;
   if (path != 0 && path != 4) return least;
   if (path == 4) {
     int c = 1;

@@ -372,8 +372,7 @@ template <int C>
 int launch_cluster(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s) {
   const ClusterSmem L(n);
   const size_t smem = L.total;
-  QTX_CHECK_CUDA(cudaFuncSetAttribute(zinv_cluster_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      (int)smem));
+  QTX_TRY(allow_dynamic_smem(zinv_cluster_kernel<C>));
   CUtensorMap map;
   const int use_tma = make_map(&map, n, batch, A) ? 1 : 0;
   if (!use_tma) memset(&map, 0, sizeof(map));

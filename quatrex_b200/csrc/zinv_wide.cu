@@ -234,7 +234,7 @@ template <int NB>
 int run_wide(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, Scratch sc,
              cudaStream_t s) {
   const size_t psm = panel_smem<NB>(n);
-  QTX_CHECK_CUDA(cudaFuncSetAttribute(zw_panel<NB>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)psm));
+  QTX_TRY(allow_dynamic_smem(zw_panel<NB>));
   const int panels = (n + NB - 1) / NB;
   ProfScope prof(QTX_KERNEL_ZINV, 8.0 * (double)n * n * n * (double)batch, s, 4 * panels + 3);
   if (A.p != X.p || A.ld != X.ld || A.stride != X.stride) {
