@@ -153,19 +153,20 @@ int qtx_zinv_batched_ws(int n, int64_t batch, qtx_mat a, qtx_mat x, int* info, v
                         size_t workspace_bytes, qtx_stream stream);
 
 /* Inverse path of every inverse in this process: 0 automatic (default),
- * 1 one CTA per matrix (two for 400 < n <= 512), 2 multi-CTA (workspace-backed
+ * 1 one CTA per matrix (two for 432 < n <= 512), 2 multi-CTA (workspace-backed
  * calls, n > 512 in the automatic choice), 3 one thread-block cluster of
  * ceil(n / 32) CTAs per matrix holding it in distributed shared memory
  * (n <= 256; loaded with TMA), 4 the path-1 kernel as a cluster of C CTAs per
  * matrix that split its columns (n <= 512; C the largest of 2, 4, 8 leaving 32
  * columns per CTA). Automatic: the distributed-shared-memory cluster for
  * n <= 256 while batch x ceil(n / 32) is at most the SM count (half of it above
- * n = 128); else up to n = 512 the column split with the largest C <= 8 (any
+ * n = 128); else up to n = 103 one CTA per matrix, which stays in its shared
+ * memory; else up to n = 512 the column split with the largest C <= 8 (any
  * number) for which batch x C fits the SM count and every cluster is
- * co-resident (C = 1 at full batches, the matrix staying in shared memory up to n = 100); above n = 512
- * the multi-CTA path for batches up to half the SM count. All paths use the
- * same pivot rule; paths 1, 3 and 4 give bit-identical results up to n = 256,
- * 1 and 4 up to n = 512. A tuning and test knob; no reference counterpart. */
+ * co-resident (C = 1 at full batches); above n = 512 the multi-CTA path for
+ * batches up to half the SM count. All paths use the same pivot rule; paths 1,
+ * 3 and 4 give bit-identical results up to n = 256, 1 and 4 up to n = 512. A
+ * tuning and test knob; no reference counterpart. */
 int qtx_set_inverse_path(int mode);
 /* 1 if a bounded wait inside the cluster inverse timed out since the last
  * call (the flag is cleared; those results are invalid), 0 if not, < 0 on

@@ -1,26 +1,27 @@
 // Batched complex128 matrix inverse: blocked Gauss-Jordan with partial
-// pivoting, one CTA per matrix.
+// pivoting, a CTA or a small cluster per matrix.
 //
 // Replaces the batched inverse of qttools kernels/linalg/inv.py:6-40
 // (numpy.linalg.inv on CPU; cupy.linalg.solve(a, I) -> cuBLAS batched
 // getrf/getrs on NVIDIA GPUs). Every diagonal Schur-complement block of the
-// RGF forward sweep and every Sancho-Rubio step inverts through here.
+// RGF forward sweep and every Sancho-Rubio step inverts through here, or through
+// the kernels of zinv_cluster.cu (n <= 256, few matrices) and zinv_wide.cu
+// (n > 512, few matrices), to which zinv_ex dispatches.
 //
-// Algorithm (in place in X, n x n, panel width NB):
-//   for each panel K = [k0, k0 + NB):
-//     1. stage the n x NB panel X[:, K] in shared memory;
-//     2. factor it column by column: pivot = argmax_{r >= k} |Re|+|Im|
-//        (LAPACK izamax measure), swap, scale the pivot row by 1/pivot
-//        (Smith's complex division), eliminate every other row. Afterwards
-//        the panel holds T[:, K], where T is the Gauss-Jordan transform of
-//        this panel: T = [A_KK^-1 ; -A_RK A_KK^-1] in block form;
-//     3. apply the panel's row swaps to all other columns (global memory);
-//     4. update every other column tile J:
-//          X[:, J] = [0 ; X[R, J]] + T[:, K] X[K, J]
-//        a n x |J| x NB complex GEMM on the FP64 tensor pipe (DMMA);
-//     5. write the panel back.
-//   Finally undo the column permutation (pivots applied in reverse order).
-// Total work n^3 complex multiply-adds = 8 n^3 real flops.
+// Three kernels by block size, one scheme (in place in X, panels K of NB columns):
+//   1. factor X[:, K] column by column: pivot = argmax_{r >= k} |Re|+|Im| (the
+//      izamax measure of LAPACK), eliminate every other row. Afterwards the
+//      panel holds T, the Gauss-Jordan transform of this panel:
+//      T = [A_KK^-1 ; -A_RK A_KK^-1] in block form;
+//   2. with the panel's row interchanges, update all other columns J:
+//        X[:, J] = [0 ; X[R, J]] + T X[K, J]
+//      a complex GEMM on the FP64 tensor pipe (DMMA).
+// Finally the columns are permuted back. n^3 complex multiply-adds = 8 n^3 flops.
+//   n <= 512:  zinv3_kernel, panel in registers, interchanges folded into the
+//              update, columns split over up to 8 CTAs, or (n <= 103) the matrix
+//              resident in shared memory;
+//   n <= 720:  zinv2_kernel, panel and pivot rows in shared memory;
+//   n <= 1024: zinv_kernel, one 32-column tile of the pivot rows at a time.
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -33,6 +34,8 @@ namespace cg = cooperative_groups;
 namespace qtx {
 namespace {
 
+// 720 < n <= 1024, one CTA per matrix: the row interchanges of a panel are staged
+// with each 32-column tile of the update.
 constexpr int THREADS = 256;
 constexpr int WARPS = THREADS / 32;
 constexpr int JW = 32;  // column-tile width of the trailing update
@@ -707,7 +710,7 @@ int launch2(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* acti
 // A cluster barrier ends the panel when C > 1 (other CTAs read the next panel
 // through L2). Finally the columns are gathered in the order of the pivoting.
 //
-// RES: the matrix stays in shared memory from load to store (n <= 100, one
+// RES: the matrix stays in shared memory from load to store (n <= 103, one
 // CTA); otherwise each panel is a pass over the matrix in L2 / HBM, which at
 // 256 x 256 x 148 moves 5 GB a launch, about half of its time.
 struct Smem3 {
@@ -967,8 +970,13 @@ int launch3(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* acti
 
 // Clusters of c CTAs of the column-split kernel that the GPU runs at once.
 int active_clusters(int n, int c) {
-  static thread_local std::vector<std::pair<int64_t, int>> cache;  // (n * 16 + c, clusters)
-  const int64_t key = (int64_t)n * 16 + c;
+  static thread_local std::vector<std::pair<int64_t, int>> cache;  // ((device, n, c), clusters)
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  const int64_t key = ((int64_t)dev << 32) + (int64_t)n * 16 + c;
   for (auto& e : cache)
     if (e.first == key) return e.second;
   cudaLaunchConfig_t cfg;
@@ -998,7 +1006,8 @@ bool fits_resident(int n) { return n <= 128 && Smem3::bytes(n, 1, true) <= kMaxD
 
 // Column split of the n <= 512 kernel: the largest C <= 8 with batch x C within
 // the SM count, at least 32 columns per CTA, and all batch clusters
-// co-resident; at least two where one CTA's pivot rows and transform do not fit.
+// co-resident; at least two where one CTA's pivot rows and transform do not fit
+// (n > 432).
 // (Powers of two alone left 64 of 148 SMs idle at n = 512, batch 42: 5.0 ms
 // against 3.6 with C = 3.) Inverse path 4 forces the largest power of two
 // that the block size allows.
@@ -1018,11 +1027,13 @@ int column_split(int n, int64_t batch) {
 }
 
 int launch_split(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s) {
-  const int c = column_split(n, batch);
+  // A resident block is not split: n = 100, batch 74 157 us against 163 us in
+  // two CTAs through L2.
   if (inverse_path() != 4 && fits_resident(n)) {
     if (n <= 64) return launch3<256, 2, true>(n, batch, A, X, info, active, s, 1);
     return launch3<512, 4, true>(n, batch, A, X, info, active, s, 1);
   }
+  const int c = column_split(n, batch);
   if (n <= 128) return launch3<512, 4, false>(n, batch, A, X, info, active, s, c);
   if (n <= 256) return launch3<512, 8, false>(n, batch, A, X, info, active, s, c);
   return launch3<512, 16, false>(n, batch, A, X, info, active, s, c);

@@ -1,6 +1,6 @@
 """The batched inverse at the edges of its paths: panels of 16 columns, the
-shared-memory-resident limit (n = 100), the row and column splits, blocks of
-257-512 columns, and pivot ties.
+shared-memory-resident limit (n = 103), the row and column splits, blocks of
+257-512 columns (two CTAs at least from 433 on), and pivot ties.
 
 Gauss-Jordan with partial pivoting leaves a residual of a few n u |A||X| for
 well-conditioned blocks (u = 1.1e-16); the bound taken is 8 n u relative to
@@ -38,8 +38,8 @@ def _residual(a, x):
     return float((a @ x - eye).norm() / (a.norm() * x.norm()))
 
 
-@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 31, 33, 64, 65, 96, 100, 101, 128, 129, 200, 256, 257, 400, 416,
-                               417, 512])
+@pytest.mark.parametrize("n", [1, 2, 15, 16, 17, 31, 33, 64, 65, 96, 100, 101, 102, 103, 104, 128, 129, 200, 256,
+                               257, 400, 416, 417, 432, 433, 512])
 @pytest.mark.parametrize("batch", [2, 40])
 def test_inverse_sizes_and_paths(cuda_device, n, batch):
     rng = np.random.default_rng(n)

@@ -1,7 +1,7 @@
 """Column-split inverse: the one-CTA Gauss-Jordan kernel launched as a
 cluster of C CTAs per matrix, each factoring every panel itself and
 updating its own range of columns (replaces the batched inverse of qttools
-kernels/linalg/inv.py:6-40 for small batches of blocks up to 400 wide).
+kernels/linalg/inv.py:6-40 for small batches of blocks up to 512 wide).
 
 Every CTA of a cluster runs the same panel arithmetic on the same data, and
 each column is updated by exactly one CTA with the same instruction sequence
@@ -94,7 +94,7 @@ def test_split_in_place_strided_and_permuted(cuda_device, path, n):
 
 def test_split_singular_report_and_automatic_choice(cuda_device, path):
     """A zero column reports its 1-based index from every path; at a small
-    batch the automatic choice (column split for n <= 400) gives the
+    batch the automatic choice (column split for 103 < n <= 512) gives the
     single-CTA bits."""
     n, B = 256, 16
     rng = np.random.default_rng(3)
