@@ -280,10 +280,16 @@ __global__ void __launch_bounds__(RT) reduce_kernel(int m, int n, int64_t batch,
   if (rank == 0 && threadIdx.x == 0) done(b, tot);
 }
 
+// |z|. x^2 + y^2 over- and underflows only where the square of |z| that is summed
+// does too; an infinite part counts as infinite beside a NaN, as in hypot: an
+// energy that overflows has not converged, and the batch-wide maximum skips NaN.
+__device__ __forceinline__ double modulus(z64 z) {
+  return isinf(z.x) || isinf(z.y) ? INFINITY : sqrt(z.x * z.x + z.y * z.y);
+}
 // (|x| + |y|)^2; delta[b] = sqrt(sum) / 2.
 struct DeltaTerm {
   __device__ __forceinline__ void operator()(z64 a, z64 w, double (&s)[1]) const {
-    const double v = sqrt(a.x * a.x + a.y * a.y) + sqrt(w.x * w.x + w.y * w.y);
+    const double v = modulus(a) + modulus(w);
     s[0] += v * v;
   }
 };
