@@ -24,6 +24,8 @@
 // one lane 1570 / 2020 / 2240, with two 1350 / 1660 / 2450 (half the row to
 // publish and to update, twice the warps to search), so two up to n = 128. (Two
 // lanes, five shuffle rounds and an unrolled loop took about 3000 at n = 256.)
+// These are with four-instruction eliminations; with the six of gj_eliminate they
+// are about 50, 30 and 290 more.
 // Measured beside it, alone, at n = 64 / 256: one lane 1120 / 1455, every warp
 // publishing its candidate row ahead of a single barrier 1130 / 2340, whole
 // columns in a warp with the multipliers published 1100 / 2440.
@@ -78,12 +80,18 @@ __device__ __forceinline__ double gj_abs1(z64 z) { return fabs(z.x) + fabs(z.y);
 
 // a b and v - m q with the roundings spelled out: every instantiation of the
 // factorization gives the same bits, so one block's inverse does not depend on
-// the path that the batch size selects.
+// the path that the batch size selects. The product is formed before it is
+// subtracted: adding its two real products to v one after another (four fma
+// instead of six instructions) rounds at the size of v twice and made the error
+// of the inverse 1.05 to 1.19 times as large at n = 16, its residual 1.02 to 1.2
+// times up to n = 256. It costs 1 to 7 % of the inverse's time (64 x 32 61 -> 62.5
+// us, 128 x 32 150.9 both, 256 x 148 1.33 -> 1.37 ms, 256 x 18 0.536 -> 0.573 ms).
 __device__ __forceinline__ z64 gj_mul(z64 a, z64 b) {
   return make_double2(fma(a.x, b.x, -__dmul_rn(a.y, b.y)), fma(a.x, b.y, __dmul_rn(a.y, b.x)));
 }
 __device__ __forceinline__ z64 gj_eliminate(z64 v, z64 m, z64 q) {
-  return make_double2(fma(-m.x, q.x, fma(m.y, q.y, v.x)), fma(-m.x, q.y, fma(-m.y, q.x, v.y)));
+  const z64 t = gj_mul(m, q);
+  return make_double2(__dsub_rn(v.x, t.x), __dsub_rn(v.y, t.y));
 }
 
 // Shared memory of gj_factor_panel.
