@@ -541,7 +541,7 @@ def run_ours(args, world, rank, local):
             "ms_per_step": float(tm.item()) / args.steps,
             "speedup_vs_fp64": ms_max / float(tm.item()),
             "dtype": "c64 storage; tcgen05 split-TF32 products, FP32 accumulation; FP64 inverses and OBC",
-            "roofline": {"bound": "tensor", "kernel": "cgemm_tc (tcgen05 kind::tf32, 12 MMAs per complex K step)",
+            "roofline": {"bound": "tensor", "kernel": "cgemm_tc (tcgen05 kind::tf32, six MMAs of N = 128 per complex K step)",
                          "achieved": ach, "peak": tf32_peak, "unit": "TFLOP/s (complex as-written 8mnk)",
                          "frac": (ach / tf32_peak) if (ach and tf32_peak) else None,
                          "peak_source": "measured cuBLAS FP32 GEMM with TF32 tensor cores 8192^3 on this GPU",
@@ -644,9 +644,9 @@ def run_ours(args, world, rank, local):
                     "peak_source": "measured cuBLAS FP64 (max of DGEMM 8192^3, ZGEMM 4096^3) on this GPU; "
                                    "no FP64 entry in MEASURED_PEAKS.json",
                     "peak_detail": peak, "traffic": _ncu_traffic(),
-                    "traffic_source": "stored ncu capture of one full-batch launch "
-                                      "(profiles/zgemm_traffic.txt: dram__bytes_read.sum + dram__bytes_write.sum), "
-                                      "not measured in this run",
+                    "traffic_source": "stored ncu capture of one launch of one product per entry of a full batch "
+                                      "(profiles/zgemm_traffic.txt: dram__bytes_read.sum + dram__bytes_write.sum; "
+                                      "the timed launches hold up to four products), not measured in this run",
                     "launches": gemm_n}
     elif main_prec == "emulated":
         S = args.emulated_slices
@@ -657,7 +657,7 @@ def run_ours(args, world, rank, local):
                     "peak_source": "measured cuBLASLt int8 GEMM 8192^3 (torch._int_mm) on this GPU",
                     "fp64_equivalent_tflops": achieved, "traffic": None, "launches": gemm_n}
     else:
-        roofline = {"bound": "tensor", "kernel": "cgemm_tc (tcgen05 kind::tf32, 12 MMAs per complex K step)",
+        roofline = {"bound": "tensor", "kernel": "cgemm_tc (tcgen05 kind::tf32, six MMAs of N = 128 per complex K step)",
                     "achieved": achieved, "peak": tf32_peak, "unit": "TFLOP/s (complex as-written 8mnk)",
                     "frac": (achieved / tf32_peak) if achieved and tf32_peak else None,
                     "peak_source": "measured cuBLAS FP32 GEMM with TF32 tensor cores 8192^3 on this GPU",

@@ -23,7 +23,7 @@
 //    256^3 x 64 244 -> 208 us, 288^3 x 24 178 -> 119 us, 128^3 x 16 24 -> 12.5
 //    us, 160^3 x 100 141 -> 84 us; with an addend 519 -> 478 us at 256^3 x 148.
 //    64 x 32 and 32 x 64 tiles at three CTAs per SM and k-slices of 16 measured
-//    the same or slower at every size. 86 % DMMA + 4 % for the sums in ncu.
+//    the same or slower at every size. 84 % DMMA + 4 % for the sums in ncu.
 //  * Per k-step of 4 the three passes p1, p2, p3 are issued back to back; the
 //    real parts of the next step are loaded (8-byte loads) right after p1,
 //    which frees their registers, the imaginary parts after p2, so a load has

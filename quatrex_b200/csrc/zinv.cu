@@ -1027,7 +1027,7 @@ int column_split(int n, int64_t batch) {
 }
 
 int launch_split(int n, int64_t batch, MatRef A, MatRef X, int* info, const int* active, cudaStream_t s) {
-  // A resident block is not split: n = 100, batch 74 157 us against 163 us in
+  // A resident block is not split: n = 100, batch 74 161 us against 165 us in
   // two CTAs through L2.
   if (inverse_path() != 4 && fits_resident(n)) {
     if (n <= 64) return launch3<256, 2, true>(n, batch, A, X, info, active, s, 1);

@@ -313,8 +313,9 @@ bool zinv_prefers_cluster(int n, int64_t batch) {
   // A cluster per matrix (ceil(n / 32) CTAs) keeps it in shared memory but
   // holds C SMs for it, and the GPU co-schedules only about half of the SM
   // count in clusters of 8 (all of it in clusters of 4). Measured on B200
-  // against the column split: n = 128, batch 32 151 / 166 us; n = 64, batch 64
-  // 61 / 67 us; n = 256, batch 9 425 / 466 us but batch 18 844 / 528 us.
+  // against the kernel of zinv.cu: n = 128, batch 32 151 / 171 us (four CTAs);
+  // n = 64, batch 64 63 / 71 us (resident); n = 256, batch 9 436 / 510 us (eight
+  // CTAs) but batch 18 863 / 572 us (six).
   const int c = (n + 31) / 32;
   return batch * c * (c <= 4 ? 1 : 2) <= (int64_t)num_sms();
 }
@@ -325,8 +326,8 @@ bool zinv_prefers_wide(int n, int64_t batch) {
   // One CTA per matrix leaves SMs idle when the batch is below the SM count;
   // the multi-CTA path pays n/NB launches and a pass over the matrix per
   // panel. Up to n = 512 the column-split clusters of zinv.cu use the idle SMs
-  // instead (n = 512, batch 21 / 42 / 74: 2.2 / 3.6 / 5.8 ms against 3.9 / 5.7
-  // / 8.1 ms); above, the measured crossover on B200 is half the SM count.
+  // instead (n = 512, batch 21 / 42 / 74: 2.3 / 3.7 / 5.9 ms against 3.8 / 5.7
+  // / 8.2 ms); above, the measured crossover on B200 is half the SM count.
   const int sms = num_sms();
   return n > 512 && batch * 2 <= sms;
 }
